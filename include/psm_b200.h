@@ -69,7 +69,8 @@ typedef struct psm_result {
     uint64_t table_entries;   /* entries over all candidate-edge tables         */
     uint64_t alg_bytes;       /* algorithmic bytes read by the intersections    */
     uint64_t donations;       /* work-stealing donations during enumeration     */
-    uint32_t overtime;        /* 1 if the time limit was hit                    */
+    uint32_t overtime;        /* 1 if the time limit was hit (or an uncapped count
+                                 passed 2^64 - 1: count is then that value)     */
     uint32_t filter_ok;       /* 0 if a candidate set came out empty            */
     uint32_t status;          /* psm_status of this query                       */
     uint32_t reserved;

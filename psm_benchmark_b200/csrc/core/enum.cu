@@ -18,6 +18,9 @@
 //    the other rows and checks it against same-label earlier vertices; a
 //    ballot compacts the survivors. The last two depths are fused: each lane
 //    takes one candidate of depth n-2 and counts its completions itself;
+//  - query vertices without later neighbours in the matching order are not
+//    branched on: their candidates are counted and multiplied (QState::ord,
+//    weigh_prefix). The depths below are the walked ones;
 //  - initial work: the edges of the first candidate-edge table (pairs of
 //    depth-0 / depth-1 candidates) of every query of the launch, handed out
 //    in chunks by one atomic ticket; queries of up to three vertices hand out
@@ -98,6 +101,13 @@ constexpr u32 BM_WORDS = PSM_CACHE_BM_BITS / 32;
 constexpr u32 SLOT_WORDS = CACHE_CAP + BM_WORDS;
 constexpr u32 WARP_CACHE_WORDS = PSM_MAXQ * SLOT_WORDS + PSM_MEMO_CAP;  // slots + weight memo
 constexpr u32 NO_ROW = 0xFFFFFFFFu;
+// Loop steps of a search between two periodic() calls. Where counted vertices
+// multiply, a prefix may stand for 1e6 embeddings, so a capped query's end has
+// to be seen sooner, and a local count of cap / 8192 is published at once: 12-
+// vertex queries that overshot a cap of 1e9 by 10-4000x took 0.5-1.5 ms, now
+// 0.3-0.4 ms.
+constexpr u32 STEPS = 32;
+constexpr u32 STEPS_WEIGHTED = 16;
 constexpr u32 LONG_ROW = 24;     // per-lane binary-search walks longer than this go to the warp
 constexpr u32 LONG_BM_ROW = 96;  // per-lane bitmap walks longer than this go to the warp
 // With only `act` lanes holding a candidate, a lane's walk costs the warp its
@@ -127,15 +137,25 @@ struct WarpStack {
     u32 vid[PSM_MAXQ];
     u32 cur[PSM_MAXQ];
     u32 end[PSM_MAXQ];
-    u32 drv[PSM_MAXQ];
-    u32 cn[PSM_MAXQ];
-    u32 ci[PSM_MAXQ];
-    u32 flg[PSM_MAXQ];
+    uint8_t drv[PSM_MAXQ];
+    uint8_t cn[PSM_MAXQ];
+    uint8_t ci[PSM_MAXQ];
+    uint8_t flg[PSM_MAXQ];
     u32 olo[PSM_MAXQ];
     u32 ohi[PSM_MAXQ];
     u32 clen[PSM_MAXQ];
     u32 clo[PSM_MAXQ];
     u32 csum[PSM_MAXQ];  // total length of the rows behind S (algorithmic bytes)
+    // Counted vertices (QState::ord), for the current prefix:
+    u64 bytes;          // algorithmic bytes and candidates examined by the task so far
+    u64 calls;
+    u64 big;            // a local count this large is published at once
+    u32 svalid;         // counted places whose candidates (sn) and row bytes (sby) are current
+    u32 sn[PSM_MAXQ];
+    u64 sby[PSM_MAXQ];
+    u64 late;           // product of the counts after the last walked depth
+    u64 late_by;        // algorithmic bytes of their intersections
+    u64 W[PSM_MAXQ];    // by walked depth: product of the counts up to it
     u32 chunk[PSM_MAXQ][32];
 };
 
@@ -207,6 +227,7 @@ __device__ void release_caches(const QState& q, WarpStack* ws) {
     __syncwarp();
     if (lane_id() == 0) {
         ws->cvalid = 0;
+        ws->svalid = 0;
         ws->cover = 0;
         ws->cadj = 0;
     }
@@ -221,7 +242,7 @@ __device__ void release_caches(const QState& q, WarpStack* ws) {
 // caching is off, or the intersection has more than CACHE_CAP entries; the
 // level then intersects the table rows directly.
 template <u32 IS>
-__device__ bool ensure_cache(const QState& q, u32 d, WarpStack* ws, u64& bytes) {
+__device__ bool ensure_cache(const QState& q, u32 d, WarpStack* ws) {
     const u32 cm = q.cmask[d];
     if (cm == 0 || ws->cbuf == nullptr) return false;
     const u32 bit = 1u << d;
@@ -307,9 +328,9 @@ __device__ bool ensure_cache(const QState& q, u32 d, WarpStack* ws, u64& bytes) 
         __syncwarp();
     }
     if (!over && ((q.bm_depths >> d) & 1u)) set_bits(q, ws, d);
-    if (q.memo_ok && d + 2 == q.n_enum) {
+    if (q.memo_ok && d + 2 == q.walk) {
         // the weight memo belongs to S_d: start it afresh
-        const u32 nl = q.cnt[q.order[d + 1]];
+        const u32 nl = q.cnt[q.ord[d + 1]];
         for (u32 i = lane; i < nl; i += 32) ws->memo[i] = 0u;
         __syncwarp();
         if (lane == 0) ws->rsum_ok = 0;
@@ -340,7 +361,7 @@ __device__ __forceinline__ bool walk_r_with_bitmap(const WarpStack* ws, u32 d, u
 template <u32 IS>
 __device__ __forceinline__ u32 setup_level(const QState& q, u32 d, WarpStack* ws, u64& bytes) {
     u32 flg = 0, best = 0, dlo = 0, dhi = 0, olo = 0, ohi = 0;
-    if (ensure_cache<IS>(q, d, ws, bytes)) {
+    if (ensure_cache<IS>(q, d, ws)) {
         const u32 s = ws->clen[d];
         const u32 k = q.crow[d];
         flg = LV_CACHED | LV_DRV_CACHE;
@@ -407,22 +428,45 @@ __device__ __forceinline__ u32 cand_pos(const QState& q, u32 u, u32 v) {
     return q.rank[u][b >> 5] + __popc(word & ((1u << (b & 31u)) - 1u));
 }
 
+// Marks the query stopped (cap reached); the first caller stamps the time.
+__device__ __forceinline__ void cap_reached(QState& q) {
+    if (atomicExch(&q.stop, 1u) == 0) q.done_ns = global_timer_ns();
+}
+
+// The count passed 2^64 - 1 (counted vertices multiply): a capped query is
+// certainly at its cap, an uncapped one ends as partial.
+__device__ void count_overflow(QState& q) {
+    atomicExch(&q.sat, 1u);
+    if (!q.cap) atomicExch(&q.overtime, 1u);
+    cap_reached(q);
+}
+
+// Adds a warp's local count to the query's (one lane); returns the new total.
+__device__ __forceinline__ u64 add_count(QState& q, u64 count) {
+    const u64 old = atomicAdd((unsigned long long*)&q.count, (unsigned long long)count);
+    const u64 total = old + count;
+    if (total < old) count_overflow(q);
+    if (q.cap && total >= q.cap) cap_reached(q);
+    return total;
+}
+
+// The number a query reports: min(count, cap).
+__device__ __forceinline__ u64 clamped_count(QState& q, u64 c) {
+    if (ld_volatile_u32(&q.sat)) return q.cap ? q.cap : ~0ull;
+    return q.cap && c > q.cap ? q.cap : c;
+}
+
 // Writes a finished query's completion record (its count is final: every
 // task of the query published before the caller's counter reached zero).
 __device__ void finish_query(QState& q, QDoneRec* rec) {
     __threadfence();
     const u64 c = atomicAdd((unsigned long long*)&q.count, 0ull);
-    rec->count = q.cap && c > q.cap ? q.cap : c;
+    rec->count = clamped_count(q, c);
     rec->overtime = ld_volatile_u32(&q.overtime);
     rec->status = q.status;
     rec->done_ns = global_timer_ns();
     __threadfence_system();
     *(volatile u32*)&rec->flag = 1u;
-}
-
-// Marks the query stopped (cap reached); the first caller stamps the time.
-__device__ __forceinline__ void cap_reached(QState& q) {
-    if (atomicExch(&q.stop, 1u) == 0) q.done_ns = global_timer_ns();
 }
 
 // One lane's candidate test at depth d for driver element p (a position in
@@ -470,12 +514,12 @@ __device__ __forceinline__ bool chunk_accept(const QState& q, u32 d, u32 p, bool
 
 // Warp-level count of the candidates of the last depth d given the prefix.
 template <u32 IS>
-__device__ u64 count_last(const QState& q, u32 d, WarpStack* ws, u64& bytes, u64& calls) {
+__device__ __forceinline__ u64 count_last(const QState& q, u32 d, WarpStack* ws, u64& bytes) {
     const u32 lane = lane_id();
-    const u32 u = q.order[d];
+    const u32 u = q.ord[d];
     const u32* list_d = q.list[u];
     const u32 len = setup_level<IS>(q, d, ws, bytes);
-    calls += len;
+    if (lane == 0) ws->calls += len;
     if (len == 0) return 0;
     const u32 f = ws->flg[d];
     const u32 lo = ws->cur[d], hi = ws->end[d];
@@ -500,20 +544,92 @@ __device__ u64 count_last(const QState& q, u32 d, WarpStack* ws, u64& bytes, u64
     return c;
 }
 
+// Whether data vertex v is among the candidates of counted place s (in all of
+// its rows). Warp-uniform, every lane searches.
+__device__ bool sink_has(const QState& q, u32 s, const WarpStack* ws, u32 v) {
+    const u32 x = cand_pos(q, q.ord[s], v);
+    if (x == 0xFFFFFFFFu) return false;
+    for (u32 k = 0; k < q.nbn[s]; ++k)
+        if (!contains_u32(q.adj, row_lo(q, s, k, ws->pos), row_hi(q, s, k, ws->pos), x)) return false;
+    return true;
+}
+
+// The weight ws->W[d] of the prefix ws->pos[0, d]: the product of the counts
+// of the counted vertices before walked depth d + 1 in the matching order, each
+// less the walked vertices among its candidates. W is also the number of the
+// order's partial embeddings that this prefix stands for, so with `account`
+// the counted vertices' algorithmic bytes are added once per such partial
+// embedding. When the last walked depth comes next, the counted vertices after
+// it (independent of it) are taken too (ws->late, ws->late_by). A count is
+// kept (ws->sn, ws->sby) until a walked depth that it depends on changes.
+// Returns whether the prefix has any completion as far as is known.
+// Warp-uniform; not inlined: a query without counted vertices pays neither
+// registers nor instruction cache for it.
+template <u32 IS>
+__device__ __noinline__ bool weigh_prefix(const QState& q, u32 d, WarpStack* ws, bool account) {
+    u64 w = d ? ws->W[d - 1] : 1ull;
+    const u32 h = q.sink_hit[d];
+    if (h && w && sink_has(q, h, ws, ws->vid[d])) {
+        // one candidate of the counted place h less: h's own factor so far is
+        // its count less the earlier hits after it
+        u32 now = ws->sn[h];
+        for (u32 j = 0; j < d; ++j)
+            if (q.sink_hit[j] == h && sink_has(q, h, ws, ws->vid[j])) --now;
+        w = w / now * (now - 1u);
+    }
+    const u32 e = q.sink_beg[d + 1], end = d + 3 == q.walk ? q.n_enum : e;
+    u64 f = w, by = 0, head = 0, head_by = 0;
+    u32 s = q.sink_beg[d];
+    for (;; ++s) {
+        if (s == e) {  // the rest comes after the last walked depth
+            head = f, head_by = by;
+            f = f ? 1 : 0, by = 0;
+        }
+        if (s >= end || f == 0) break;
+        if (!((ws->svalid >> s) & 1u)) {
+            u64 rows = 0;
+            const u32 c = (u32)count_last<IS>(q, s, ws, rows);
+            __syncwarp();
+            if (lane_id() == 0) {
+                ws->sn[s] = c;
+                ws->sby[s] = rows;
+                ws->svalid |= 1u << s;
+            }
+            __syncwarp();
+        }
+        by += f * ws->sby[s];
+        f *= ws->sn[s];
+    }
+    if (s < e) head_by = by;  // no candidates: head = 0
+    __syncwarp();
+    if (lane_id() == 0) {
+        ws->W[d] = head;
+        ws->late = f;
+        ws->late_by = by;
+        if (account) ws->bytes += head_by;
+    }
+    __syncwarp();
+    return head != 0;
+}
+
 // Emits the embeddings of the last depth (original data ids, indexed by
 // query vertex) into q.emit_buf; returns how many were found.
 template <u32 IS>
-__device__ u64 emit_last(QState& q, const DevGraph& g, u32 d, WarpStack* ws, u64& bytes, u64& calls) {
+__device__ u64 emit_last(QState& q, const DevGraph& g, u32 d, WarpStack* ws) {
     const u32 lane = lane_id();
     const u32 n = d + 1;
-    const u32 u = q.order[d];
+    const u32 u = q.ord[d];
     const u32* list_d = q.list[u];
     // A capped query stops emitting as soon as the rows reach its cap (the
     // rows emitted so far are the rows counted): a stopped query emits
     // nothing more, and the chunk that crosses the cap is the warp's last.
     if (q.cap && warp_ld_volatile_u32(&q.stop)) return 0;
-    u32 blen = setup_level<IS>(q, d, ws, bytes);
-    calls += blen;
+    u64 by = 0;
+    const u32 blen = setup_level<IS>(q, d, ws, by);
+    if (lane == 0) {
+        ws->bytes += by;
+        ws->calls += blen;
+    }
     const u32 bs = ws->cur[d];
     u64 c = 0;
     for (u32 j = 0; j < blen; j += 32) {
@@ -542,7 +658,7 @@ __device__ u64 emit_last(QState& q, const DevGraph& g, u32 d, WarpStack* ws, u64
                     for (u32 i = 0; i < d; ++i) out[i] = ws->vid[i];
                     out[d] = list_d[p];
                 } else {
-                    for (u32 i = 0; i < d; ++i) out[q.order[i]] = g.orig[ws->vid[i]];
+                    for (u32 i = 0; i < d; ++i) out[q.ord[i]] = g.orig[ws->vid[i]];
                     out[u] = g.orig[list_d[p]];
                 }
             }
@@ -572,7 +688,7 @@ __device__ u64 emit_last(QState& q, const DevGraph& g, u32 d, WarpStack* ws, u64
 // one, v is not looked up.
 __device__ __forceinline__ u32 cached_exclusions(const QState& q, u32 dl, u32 v, const WarpStack* ws, bool has_row,
                                                  u32 lo, u32 hi) {
-    const u32 u = q.order[dl];
+    const u32 u = q.ord[dl];
     const u32 dp = dl - 1;
     u32 c = 0;
     for (u32 m = q.same_mask[dl]; m; m &= m - 1) {
@@ -646,7 +762,7 @@ __device__ u64 lane_last_count(const QState& q, u32 dl, bool cached, u32 p, u32 
         *defer = true;
         return 0;
     }
-    const u32 u = q.order[dl];
+    const u32 u = q.ord[dl];
     const u32 same = q.same_mask[dl];
     if (nb == 1) {
         u64 c = blen;
@@ -747,7 +863,7 @@ __device__ u64 warp_last_count(const QState& q, u32 dl, bool cached, u32 p, u32 
             b2len = hi - lo, b2lo = lo, bk2 = k;
         }
     }
-    const u32 u = q.order[dl];
+    const u32 u = q.ord[dl];
     const u32 same = q.same_mask[dl];
     const u32* list = q.list[u];
     if (IS != ISECT_BINARY && bk2 != 0xFFFFFFFFu && warp_merge_pays(IS, blen, b2len)) {
@@ -814,7 +930,7 @@ struct MemoOut {
 __device__ __forceinline__ MemoOut memo_count(const QState& q, u32 d, WarpStack* ws) {
     const u32 lane = lane_id();
     const u32 l = d + 1;
-    const u32 ud = q.order[d], ul = q.order[l];
+    const u32 ud = q.ord[d], ul = q.ord[l];
     const u32* Sd = cache_list(q, ws, d);
     const u32 sd = ws->clen[d];
     const u32* bmd = slot_bm(ws, d);
@@ -1023,7 +1139,7 @@ __device__ bool try_donate_range(EnumCtl* ctl, Slot* slots, u32 kind, u32 qi, u3
     return false;
 }
 
-// Every 16 warp steps inside a search: donate work to hungry warps, publish
+// Every STEPS warp steps inside a search: donate work to hungry warps, publish
 // the local count (so a capped query stops close to its cap) and stop on the
 // cap or the time limit. Returns true when the search must stop.
 __device__ bool periodic(QState& q, u32 qi, WarpStack* ws, u32 d, u32 d0, u32 iter, u64& count, EnumCtl* ctl,
@@ -1081,12 +1197,8 @@ __device__ bool periodic(QState& q, u32 qi, WarpStack* ws, u32 d, u32 d0, u32 it
     // the query then stops close to the cap instead of up to a share per warp
     // beyond it. Only lane 0 reads and writes near_q.
     if (lane == 0 && count >= (ws->near_q == qi ? (1ull << 10) : (1ull << 14))) {
-        unsigned long long old = atomicAdd((unsigned long long*)&q.count, count);
-        if (q.cap) {
-            const u64 total = old + count;
-            if (total >= q.cap) cap_reached(q);
-            if (total + ((u64)(gridDim.x * (blockDim.x >> 5)) << 17) >= q.cap) ws->near_q = qi;
-        }
+        const u64 total = add_count(q, count);
+        if (q.cap && total + ((u64)(gridDim.x * (blockDim.x >> 5)) << 17) >= q.cap) ws->near_q = qi;
         count = 0;
     }
     count = __shfl_sync(FULL_MASK, count, 0);
@@ -1107,66 +1219,118 @@ __device__ bool periodic(QState& q, u32 qi, WarpStack* ws, u32 d, u32 d0, u32 it
     return __shfl_sync(FULL_MASK, stop, 0) != 0;
 }
 
-// Depth-first search below the prefix ws->pos[0, d0): the level d0 has been
-// set up (driver range in ws). Returns false if the query stopped.
-template <u32 IS>
-__device__ bool dfs(const DevGraph& g, QState& q, u32 qi, u32 d0, WarpStack* ws, EnumCtl* ctl, Slot* slots, bool emit,
-                    u64& count, u64& bytes, u64& calls, u32& iter) {
+// count += c * w; false when that passes 2^64 - 1.
+__device__ __forceinline__ bool add_weighted(u64& count, u64 c, u64 w) {
+    const u64 x = c * w;
+    count += x;
+    return __umul64hi(c, w) == 0 && count >= x;
+}
+
+// Depth-first search below the prefix ws->pos[0, d0). With `enter` the walked
+// vertex of depth d0 - 1 was just placed (its weight and the level d0 are set up
+// here), otherwise the level d0 has been set up (driver range in ws). Returns
+// false if the query stopped.
+template <u32 IS, bool EMIT>
+__device__ __forceinline__ bool dfs(const DevGraph& g, QState& q, u32 qi, u32 d0, bool enter, WarpStack* ws, EnumCtl* ctl,
+                                    Slot* slots, u64& count, u32& iter) {
     const u32 lane = lane_id();
-    const u32 n = q.n_enum;
-    u32 d = d0;
+    const u32 n = q.walk;
+    const bool weights = !EMIT && n != q.n_enum;  // some vertices are counted, not walked
+    u32 d = enter ? d0 - 1 : d0;
     u64 bytes_l = 0, calls_l = 0;  // per-lane parts, summed at the end
     bool go = true;
+    const u32 every = weights ? STEPS_WEIGHTED : STEPS;
     while (true) {
-        if (d + 2 == n && !emit) {
-            // The last two depths fused: each lane takes one driver element
-            // of depth d and counts its completions at depth d + 1 on its own.
-            if (ws->cur[d] < ws->end[d] && q.memo_ok && ((ws->lvfull >> d) & 1u) &&
-                (ws->flg[d] & LV_CACHED) && ((ws->cbits >> d) & 1u) && ensure_cache<IS>(q, d + 1, ws, bytes)) {
-                // the whole level at once through the weight memo
-                const MemoOut mo = memo_count(q, d, ws);
-                count += mo.count;
-                bytes += mo.bytes;
-                calls += mo.calls;
-                __syncwarp();
-                if (lane == 0) ws->cur[d] = ws->end[d];
-                __syncwarp();
-                if ((++iter & 15u) == 0 && periodic(q, qi, ws, d, d0, iter, count, ctl, slots)) {
-                    go = false;
-                    break;
-                }
+        if (((++iter & (every - 1u)) == 0 || count >= ws->big) && periodic(q, qi, ws, d, d0, iter, count, ctl, slots)) {
+            go = false;
+            break;
+        }
+        if (enter) {
+            // below the vertex just placed at depth d
+            enter = false;
+            if (weights && !weigh_prefix<IS>(q, d, ws, true)) {
+                if (d < d0) break;
                 continue;
             }
-            if (ws->cur[d] < ws->end[d]) {
-                const u32 cur = ws->cur[d], end = ws->end[d];
-                const u32 idx = cur + lane;
-                u64 c = 0;
-                bool defer = false;
-                const u32* list_d = q.list[q.order[d]];
-                // the last depth's cache depends on depths <= d - 1 only
-                const bool cached = ensure_cache<IS>(q, d + 1, ws, bytes);
-                const bool valid = idx < end;
-                const u32 p = valid ? (d == 0 ? idx : drv_elem(q, ws, d, idx)) : 0u;
-                const bool ok = d == 0 ? valid : chunk_accept(q, d, p, valid, ws, list_d);
-                const u32 v = ok ? list_d[p] : 0u;
-                const u32 act = __popc(__ballot_sync(FULL_MASK, ok));
-                if (ok) c = lane_last_count<IS>(q, d + 1, cached, p, v, ws, bytes_l, calls_l, &defer, act);
-                count += warp_sum64(c);
-                // long intersections deferred by their lanes: whole warp each
-                u32 dm = __ballot_sync(FULL_MASK, defer);
-                while (dm) {
-                    const u32 src = __ffs(dm) - 1;
-                    dm &= dm - 1;
-                    count += warp_last_count<IS>(q, d + 1, cached, __shfl_sync(FULL_MASK, p, src),
-                                             __shfl_sync(FULL_MASK, v, src), ws);
+            u64 by = 0;
+            if (d + 2 == n) {
+                if constexpr (EMIT) {
+                    count += emit_last<IS>(q, g, d + 1, ws);
+                } else {
+                    count += count_last<IS>(q, d + 1, ws, by);
+                    if (lane == 0) ws->bytes += by;
                 }
-                calls += min(32u, end - cur);
-                __syncwarp();
-                if (lane == 0) ws->cur[d] = min(end, cur + 32u);
-                __syncwarp();
-                if ((++iter & 15u) == 0 && periodic(q, qi, ws, d, d0, iter, count, ctl, slots)) {
-                    go = false;
-                    break;
+                if (d < d0) break;
+            } else {
+                setup_level<IS>(q, d + 1, ws, by);
+                if (lane == 0) ws->bytes += weights ? by * ws->W[d] : by;
+                d += 1;
+            }
+            continue;
+        }
+        if (!EMIT && d + 2 == n) {
+            // The last two depths fused: each lane takes one driver element
+            // of depth d and counts its completions at depth d + 1 on its own.
+            if (ws->cur[d] < ws->end[d]) {
+                u64 c = 0;
+                u32 act;  // candidates of depth d in this step
+                if (q.memo_ok && ((ws->lvfull >> d) & 1u) && (ws->flg[d] & LV_CACHED) && ((ws->cbits >> d) & 1u) &&
+                    ensure_cache<IS>(q, d + 1, ws)) {
+                    // the whole level at once through the weight memo
+                    const MemoOut mo = memo_count(q, d, ws);
+                    c = mo.count;
+                    act = (u32)mo.calls;
+                    if (lane == 0) {
+                        ws->calls += mo.calls;
+                        ws->bytes += weights ? mo.bytes * ws->W[d - 1] * ws->late : mo.bytes;
+                    }
+                    __syncwarp();
+                    if (lane == 0) ws->cur[d] = ws->end[d];
+                    __syncwarp();
+                } else {
+                    const u32 cur = ws->cur[d], end = ws->end[d];
+                    const u32 idx = cur + lane;
+                    bool defer = false;
+                    const u32* list_d = q.list[q.ord[d]];
+                    // the last depth's cache depends on depths <= d - 1 only
+                    const bool cached = ensure_cache<IS>(q, d + 1, ws);
+                    const bool valid = idx < end;
+                    const u32 p = valid ? (d == 0 ? idx : drv_elem(q, ws, d, idx)) : 0u;
+                    const bool ok = d == 0 ? valid : chunk_accept(q, d, p, valid, ws, list_d);
+                    const u32 v = ok ? list_d[p] : 0u;
+                    act = __popc(__ballot_sync(FULL_MASK, ok));
+                    u64 by = 0;
+                    if (ok) c = lane_last_count<IS>(q, d + 1, cached, p, v, ws, by, calls_l, &defer, act);
+                    bytes_l += weights ? by * (ws->W[d - 1] * ws->late) : by;
+                    c = warp_sum64(c);
+                    // long intersections deferred by their lanes: whole warp each
+                    u32 dm = __ballot_sync(FULL_MASK, defer);
+                    while (dm) {
+                        const u32 src = __ffs(dm) - 1;
+                        dm &= dm - 1;
+                        c += warp_last_count<IS>(q, d + 1, cached, __shfl_sync(FULL_MASK, p, src),
+                                                 __shfl_sync(FULL_MASK, v, src), ws);
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        ws->calls += min(32u, end - cur);
+                        ws->cur[d] = min(end, cur + 32u);
+                    }
+                    __syncwarp();
+                }
+                if (weights) {
+                    // each completion stands for W x late embeddings; the vertices
+                    // counted after depth d are read once per candidate of depth d
+                    const u64 w = ws->W[d - 1], wl = w * ws->late, x = c * wl;
+                    if (lane == 0) ws->bytes += act * w * ws->late_by;
+                    count += x;
+                    if (__umul64hi(c, wl) != 0 || count < x) {
+                        if (lane == 0) count_overflow(q);
+                        go = false;
+                        break;
+                    }
+                } else {
+                    count += c;
                 }
             } else {
                 if (d == d0) break;
@@ -1180,139 +1344,136 @@ __device__ bool dfs(const DevGraph& g, QState& q, u32 qi, u32 d0, WarpStack* ws,
             if (lane == 0) {
                 ws->ci[d] += 1;
                 ws->pos[d] = p;
-                ws->vid[d] = q.list[q.order[d]][p];
+                ws->vid[d] = q.list[q.ord[d]][p];
                 const u32 inv = q.cinval[d];  // caches that depend on depth d
                 ws->cvalid &= ~inv;
                 ws->cover &= ~inv;
+                if (weights) ws->svalid &= ~q.sink_inval[d];
             }
             __syncwarp();
-            if (d + 2 == n) {
-                count += emit ? emit_last<IS>(q, g, d + 1, ws, bytes, calls) : count_last<IS>(q, d + 1, ws, bytes, calls);
-            } else {
-                d += 1;
-                setup_level<IS>(q, d, ws, bytes);
-            }
+            enter = true;
         } else if (ws->cur[d] < ws->end[d]) {
             const u32 cur = ws->cur[d], end = ws->end[d];
             const u32 idx = cur + lane;
             const bool valid = idx < end;
             const u32 p = valid ? (d == 0 ? idx : drv_elem(q, ws, d, idx)) : 0u;
-            const bool ok = d == 0 ? valid : chunk_accept(q, d, p, valid, ws, q.list[q.order[d]]);
+            const bool ok = d == 0 ? valid : chunk_accept(q, d, p, valid, ws, q.list[q.ord[d]]);
             u32 bal = __ballot_sync(FULL_MASK, ok);
             if (ok) ws->chunk[d][__popc(bal & ((1u << lane) - 1u))] = p;
-            calls += min(32u, end - cur);
             __syncwarp();
             if (lane == 0) {
+                ws->calls += min(32u, end - cur);
                 ws->cn[d] = __popc(bal);
                 ws->ci[d] = 0;
                 ws->cur[d] = min(end, cur + 32u);
             }
             __syncwarp();
-            if ((++iter & 15u) == 0 && periodic(q, qi, ws, d, d0, iter, count, ctl, slots)) {
-                go = false;
-                break;
-            }
         } else {
             if (d == d0) break;
             d -= 1;
         }
     }
-    bytes += warp_sum64(bytes_l);
-    calls += warp_sum64(calls_l);
+    bytes_l = warp_sum64(bytes_l);
+    calls_l = warp_sum64(calls_l);
+    if (lane == 0) {
+        ws->bytes += bytes_l;
+        ws->calls += calls_l;
+    }
+    __syncwarp();
     return go;
 }
 
-__device__ void publish(QState& q, u64 count, u64 bytes, u64 calls) {
+__device__ void publish(QState& q, u64 count, const WarpStack* ws) {
     if (lane_id() == 0) {
-        if (count) {
-            unsigned long long old = atomicAdd((unsigned long long*)&q.count, count);
-            if (q.cap && old + count >= q.cap) cap_reached(q);
-        }
-        if (calls) atomicAdd((unsigned long long*)&q.calls, calls);
-        if (bytes) atomicAdd((unsigned long long*)&q.alg_bytes, bytes);
+        if (count) add_count(q, count);
+        if (ws->calls) atomicAdd((unsigned long long*)&q.calls, (unsigned long long)ws->calls);
+        if (ws->bytes) atomicAdd((unsigned long long*)&q.alg_bytes, (unsigned long long)ws->bytes);
     }
 }
 
 // Runs one task (prefix positions already in ws->pos[0, d0)).
-template <u32 IS>
-__device__ void run_task(const DevGraph& g, QState* qs, const TaskHdr& t, WarpStack* ws, EnumCtl* ctl, Slot* slots,
-                         bool emit) {
+template <u32 IS, bool EMIT>
+__device__ void run_task(const DevGraph& g, QState* qs, const TaskHdr& t, WarpStack* ws, EnumCtl* ctl, Slot* slots) {
     const u32 lane = lane_id();
     QState& q = qs[t.qi];
-    const u32 n = q.n_enum;
+    const u32 n = q.walk;
+    const bool weights = !EMIT && n != q.n_enum;
     if (warp_ld_volatile_u32(&q.stop)) return;
-    u64 count = 0, bytes = 0, calls = 0;
+    u64 count = 0;
     u32 iter = 0;
+    __syncwarp();
+    if (lane == 0) {
+        ws->bytes = 0;
+        ws->calls = 0;
+        ws->W[0] = 1;  // no vertex is counted before depth 1
+        ws->big = weights && q.cap ? max(q.cap >> 13, (u64)1 << 14) : ~(u64)0;
+    }
+    __syncwarp();
     // caches start empty (release_caches ran at the end of the last task)
     if (n == 1) {  // single-vertex query: every root candidate is an embedding
         count = t.e - t.b;
-        calls = count;
-        if (emit) {
+        if constexpr (EMIT) {
             for (u32 i = t.b + lane; i < t.e; i += 32) {
                 unsigned long long r = atomicAdd((unsigned long long*)&q.emit_rows, 1ull);
-                const u32 v = q.list[q.order[0]][i];
+                const u32 v = q.list[q.ord[0]][i];
                 if (r < q.emit_cap_rows) q.emit_buf[r] = q.emit_by_depth ? v : g.orig[v];
             }
         }
-        publish(q, count, bytes, calls);
+        if (lane == 0) ws->calls = count;
+        publish(q, count, ws);
         return;
     }
-    if (t.kind == KIND_EDGES) {
-        // Pairs (root r, depth-1 candidate c) taken from the entries [b, e)
-        // of the first table T[u_0][u_1]; the root of an entry is found by
-        // walking the table's row offsets.
+    // Edge pool: pairs (root r, depth-1 candidate c) taken from the entries
+    // [b, e) of the first table T[u_0][u_1] (queries of four or more vertices);
+    // the root of an entry is found by walking the table's row offsets.
+    const bool edges = t.kind == KIND_EDGES;
+    const u32 d0 = edges ? 2u : t.d0;
+    u32 r = 0, last_r = 0xFFFFFFFFu, end = edges ? t.e : t.b + 1;
+    if (edges) {
         const u32 base = q.bn_tab[1][0];
-        const u32* list0 = q.list[q.order[0]];
-        const u32* list1 = q.list[q.order[1]];
-        const bool same01 = q.same_mask[1] & 1u;
-        u32 lo = 0, hi = q.root_cnt;  // largest r with P[base + r] <= b
-        while (hi - lo > 1) {
-            u32 mid = (lo + hi) >> 1;
+        u32 hi = q.root_cnt;  // largest r with P[base + r] <= b
+        while (hi - r > 1) {
+            u32 mid = (r + hi) >> 1;
             if (q.P[base + mid] <= t.b)
-                lo = mid;
+                r = mid;
             else
                 hi = mid;
         }
-        u32 r = lo, last_r = 0xFFFFFFFFu;
-        u32 end = t.e;
-        for (u32 e = t.b; e < end; ++e) {
+    } else {
+        // Restore the data vertices of the prefix, and its weights: the donor
+        // has accounted for them, but for the entry of a KIND_FULL task.
+        if (lane < d0) ws->vid[lane] = q.list[q.ord[lane]][ws->pos[lane]];
+        __syncwarp();
+        if (weights)
+            for (u32 d = 1; d + (t.kind == KIND_FULL ? 1u : 0u) < d0; ++d) weigh_prefix<IS>(q, d, ws, false);
+    }
+    for (u32 e = t.b; e < end; ++e) {
+        bool enter = true;
+        if (edges) {
+            const u32 base = q.bn_tab[1][0];
             while (q.P[base + r + 1] <= e) ++r;
             const u32 c = q.adj[e];
-            const u32 v0 = list0[r], v1 = list1[c];
-            calls += 1;
-            if (same01 && v0 == v1) continue;
+            const u32 v0 = q.list[q.ord[0]][r], v1 = q.list[q.ord[1]][c];
+            const bool clash = (q.same_mask[1] & 1u) && v0 == v1;
             __syncwarp();
             if (lane == 0) {
-                ws->pos[0] = r;
-                ws->vid[0] = v0;
-                ws->pos[1] = c;
-                ws->vid[1] = v1;
-                const u32 inv = q.cinval[r == last_r ? 1 : 0];
-                ws->cvalid &= ~inv;
-                ws->cover &= ~inv;
+                ws->calls += 1;
+                if (!clash) {
+                    ws->pos[0] = r;
+                    ws->vid[0] = v0;
+                    ws->pos[1] = c;
+                    ws->vid[1] = v1;
+                    const u32 x = r == last_r ? 1 : 0;
+                    const u32 inv = q.cinval[x];
+                    ws->cvalid &= ~inv;
+                    ws->cover &= ~inv;
+                    if (weights) ws->svalid &= ~q.sink_inval[x];
+                }
             }
-            last_r = r;
             __syncwarp();
-            // edge pools are built for queries of four or more vertices
-            setup_level<IS>(q, 2, ws, bytes);
-            if (!dfs<IS>(g, q, t.qi, 2, ws, ctl, slots, emit, count, bytes, calls, iter)) break;
-            if (e + 2 < end) try_donate_range(ctl, slots, KIND_EDGES, t.qi, 0, e + 1, end, 0, ws, 2u);
-        }
-        release_caches(q, ws);
-        publish(q, count, bytes, calls);
-        return;
-    }
-    // Restore the data vertices of the prefix.
-    if (lane < t.d0) ws->vid[lane] = q.list[q.order[lane]][ws->pos[lane]];
-    __syncwarp();
-    const u32 d0 = t.d0;
-    if (t.kind == KIND_FULL && d0 + 1 == n) {
-        // donated entry whose children are the last depth
-        count += emit ? emit_last<IS>(q, g, d0, ws, bytes, calls) : count_last<IS>(q, d0, ws, bytes, calls);
-    } else {
-        if (t.kind == KIND_FULL) {
-            setup_level<IS>(q, d0, ws, bytes);
-        } else {
+            if (clash) continue;
+            last_r = r;
+        } else if (t.kind == KIND_RANGE) {
             // a donated driver range: rebuild the level the donor had (its
             // cache is a function of the prefix, so the range indexes the
             // same array here)
@@ -1321,11 +1482,9 @@ __device__ void run_task(const DevGraph& g, QState* qs, const TaskHdr& t, WarpSt
             if (flg & LV_CACHED) {
                 // the donor's flags need what the donor had: the cache, and
                 // its bitmap when S is tested through it
-                if (!ensure_cache<IS>(q, d0, ws, bytes) || ((flg & LV_OTHER_BM) && !((ws->cbits >> d0) & 1u))) {
+                if (!ensure_cache<IS>(q, d0, ws) || ((flg & LV_OTHER_BM) && !((ws->cbits >> d0) & 1u))) {
                     if (lane == 0) atomicExch(&ctl->error, 1u);
-                    release_caches(q, ws);
-                    publish(q, count, bytes, calls);
-                    return;
+                    break;
                 }
                 if ((flg & LV_OTHER) && !(flg & LV_OTHER_BM)) {
                     if (flg & LV_DRV_CACHE) {
@@ -1339,21 +1498,23 @@ __device__ void run_task(const DevGraph& g, QState* qs, const TaskHdr& t, WarpSt
             __syncwarp();
             if (lane == 0) {
                 ws->lvfull &= ~(1u << d0);  // a part of the donor's level
-                ws->flg[d0] = flg;
+                ws->flg[d0] = (uint8_t)flg;
                 ws->cur[d0] = t.b;
                 ws->end[d0] = t.e;
-                ws->drv[d0] = k;
+                ws->drv[d0] = (uint8_t)k;
                 ws->olo[d0] = olo;
                 ws->ohi[d0] = ohi;
                 ws->cn[d0] = 0;
                 ws->ci[d0] = 0;
             }
             __syncwarp();
+            enter = false;
         }
-        dfs<IS>(g, q, t.qi, d0, ws, ctl, slots, emit, count, bytes, calls, iter);
+        if (!dfs<IS, EMIT>(g, q, t.qi, d0, enter, ws, ctl, slots, count, iter)) break;
+        if (edges && e + 2 < end) try_donate_range(ctl, slots, KIND_EDGES, t.qi, 0, e + 1, end, 0, ws, 2u);
     }
     release_caches(q, ws);
-    publish(q, count, bytes, calls);
+    publish(q, count, ws);
 }
 
 // Initial pool: ticket -> (query, unit range); grab_prefix[i] = grabs of the
@@ -1428,10 +1589,10 @@ __device__ bool take_initial(EnumCtl* ctl, const u32* grab_prefix, const PoolInf
     return true;
 }
 
-template <u32 IS>
+template <u32 IS, bool EMIT>
 __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, 3) enum_kernel(DevGraph g, QState* qs, EnumCtl* ctl,
                                                                     Slot* slots, const u32* grab_prefix,
-                                                                    const PoolInfo* pools, int emit, u32* cache) {
+                                                                    const PoolInfo* pools, u32* cache) {
     __shared__ WarpStack stacks[WARPS_PER_BLOCK];
     WarpStack* ws = &stacks[threadIdx.x >> 5];
     const u32 lane = lane_id();
@@ -1442,6 +1603,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, 3) enum_kernel(DevGraph 
         ws->rsum_ok = 0;
         ws->lvfull = 0;
         ws->cvalid = 0;
+        ws->svalid = 0;
         ws->cover = 0;
         ws->cbits = 0;
         ws->cadj = 0;
@@ -1458,7 +1620,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, 3) enum_kernel(DevGraph 
             if (hungry && lane == 0) atomicSub(&ctl->hungry, 1u);
             hungry = false;
             spins = 0;
-            run_task<IS>(g, qs, t, ws, ctl, slots, emit != 0);
+            run_task<IS, EMIT>(g, qs, t, ws, ctl, slots);
             ++ntasks;
             __syncwarp();
             if (lane == 0) {
@@ -1583,12 +1745,12 @@ __global__ void enum_init_kernel(QState* qs, u32 nq, EnumCtl* ctl, Slot* slots, 
     for (u32 i = threadIdx.x; i < QCAP; i += blockDim.x) slots[i].seq = i;
 }
 
-__global__ void gather_kernel(const QState* qs, u32 nq, DevResult* out) {
+__global__ void gather_kernel(QState* qs, u32 nq, DevResult* out) {
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += gridDim.x * blockDim.x) {
-        const QState& q = qs[i];
+        QState& q = qs[i];
         DevResult r;
-        r.count = q.cap && q.count > q.cap ? q.cap : q.count;
-        r.count_internal = q.count;
+        r.count = clamped_count(q, q.count);
+        r.count_internal = q.sat ? ~0ull : q.count;
         r.calls = q.calls;
         r.alg_bytes = q.alg_bytes;
         r.memory_bytes = q.memory_bytes;
@@ -1606,7 +1768,7 @@ size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 }  // namespace
 
-cudaError_t psm_launch_gather(const QState* qs, u32 nq, DevResult* out, cudaStream_t st) {
+cudaError_t psm_launch_gather(QState* qs, u32 nq, DevResult* out, cudaStream_t st) {
     u32 blocks = (nq + 255) / 256;
     gather_kernel<<<blocks ? blocks : 1, 256, 0, st>>>(qs, nq, out);
     return cudaGetLastError();
@@ -1637,17 +1799,18 @@ cudaError_t psm_launch_enum(const DevGraph& g, QState* qs, u32 nq, void* scratch
                                          (u32)blocks * WARPS_PER_BLOCK, budget_ns, max(1u, grabs_per_warp));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    // one instantiation per intersection variant: the merge paths cost the
-    // binary-search one nothing (registers, instruction cache)
+    // one instantiation per intersection variant, and for emission: what a
+    // launch does not run costs it neither registers nor instruction cache
+    // (158 -> 102 B of spill stores in the counting kernel; a query bound by
+    // its node visits 153 -> 148 ms)
+    void (*kernel)(DevGraph, QState*, EnumCtl*, Slot*, const u32*, const PoolInfo*, u32*);
     if (isect == ISECT_AUTO)
-        enum_kernel<ISECT_AUTO><<<blocks, WARPS_PER_BLOCK * 32, 0, st>>>(g, qs, ctl, slots, grab_prefix, pools, emit,
-                                                                        cache);
+        kernel = emit ? enum_kernel<ISECT_AUTO, true> : enum_kernel<ISECT_AUTO, false>;
     else if (isect == ISECT_MERGE)
-        enum_kernel<ISECT_MERGE><<<blocks, WARPS_PER_BLOCK * 32, 0, st>>>(g, qs, ctl, slots, grab_prefix, pools,
-                                                                         emit, cache);
+        kernel = emit ? enum_kernel<ISECT_MERGE, true> : enum_kernel<ISECT_MERGE, false>;
     else
-        enum_kernel<ISECT_BINARY><<<blocks, WARPS_PER_BLOCK * 32, 0, st>>>(g, qs, ctl, slots, grab_prefix, pools,
-                                                                          emit, cache);
+        kernel = emit ? enum_kernel<ISECT_BINARY, true> : enum_kernel<ISECT_BINARY, false>;
+    kernel<<<blocks, WARPS_PER_BLOCK * 32, 0, st>>>(g, qs, ctl, slots, grab_prefix, pools, cache);
     return cudaGetLastError();
 }
 
@@ -1657,7 +1820,7 @@ cudaError_t psm_enum_max_blocks(int* blocks) {
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, enum_kernel<ISECT_BINARY>, WARPS_PER_BLOCK * 32, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, enum_kernel<ISECT_BINARY, false>, WARPS_PER_BLOCK * 32, 0);
     if (e != cudaSuccess) return e;
     *blocks = sms * (per_sm < 1 ? 1 : per_sm);
     return cudaSuccess;

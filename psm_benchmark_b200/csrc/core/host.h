@@ -104,7 +104,7 @@ cudaError_t psm_launch_enum(const DevGraph& g, QState* qs, u32 nq, void* scratch
                             int emit, int blocks, u32* cache, QDoneRec* done, u32 exit_keep, cudaStream_t st,
                             u32 grabs_per_warp = 8, u32 isect = 0);
 cudaError_t psm_enum_max_blocks(int* blocks);
-cudaError_t psm_launch_gather(const QState* qs, u32 nq, DevResult* out, cudaStream_t st);
+cudaError_t psm_launch_gather(QState* qs, u32 nq, DevResult* out, cudaStream_t st);
 cudaError_t psm_enum_read_ctl(void* scratch, EnumStats* out, cudaStream_t st);
 // Split form for callers with pinned staging: queue the control block's copy
 // on the stream, then read the stats once the stream has synchronised.

@@ -65,6 +65,7 @@ __global__ void reset_counts_kernel(QState* q, u64 cap) {
     q->stop = 0;
     q->overtime = 0;
     q->emit_rows = 0;
+    q->sat = 0;
     q->cap = cap;
 }
 
@@ -116,12 +117,14 @@ extern "C" int psm_run_recount_noalloc(psm_run* run, uint64_t cap, double time_l
                             ri.enum_blocks, nullptr, nullptr, 0, ri.stream, 8u, ri.isect);
     u64 got = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&got, &ri.dq->count, sizeof(u64), cudaMemcpyDeviceToHost, ri.stream);
-    u32 ov = 0;
+    u32 ov = 0, sat = 0;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&sat, &ri.dq->sat, sizeof(u32), cudaMemcpyDeviceToHost, ri.stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&ov, &ri.dq->overtime, sizeof(u32), cudaMemcpyDeviceToHost, ri.stream);
     EnumStats es{};
     if (e == cudaSuccess) e = psm_enum_read_ctl(scratch, &es, ri.stream);  // synchronises the stream
     if (e != cudaSuccess) return psm_fail(PSM_ERR_CUDA, std::string("recount_noalloc: ") + cudaGetErrorString(e));
     if (es.error) return psm_fail(PSM_ERR_INTERNAL, "recount_noalloc: enumeration wait gave up");
+    if (sat) got = ~0ull;  // the count passed 2^64 - 1
     *count = cap && got > cap ? cap : got;
     if (overtime) *overtime = ov;
     return ov ? psm_fail(PSM_ERR_TIMEOUT, "time limit reached") : PSM_OK;

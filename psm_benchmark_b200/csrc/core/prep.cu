@@ -1006,18 +1006,111 @@ __device__ void cfl_order_select(QState& q, const u32* pw) {
     if (cnt != n) q.status = PSM_DEV_INTERNAL;
 }
 
+// Chooses the counted vertices of a query (QState::ord) and orders the
+// enumerator's depths. A vertex is counted instead of walked when
+//  - none of its neighbours comes later in the matching order (its candidates
+//    then only multiply the completions; the order's last vertex is always
+//    counted, by the lanes of the fused last two depths, and the first two
+//    stay walked: the initial pool hands them out);
+//  - no other counted vertex has its label (two of one label would exclude
+//    each other; a walked vertex of its label is handled: sink_hit);
+//  - it neither neighbours nor shares the label of the last walked vertex,
+//    whose candidates the lanes try side by side;
+//  - the product of the counted vertices' candidate counts stays below 2^52,
+//    so that a weight never overflows.
+// At least three walked depths and the last vertex remain (the initial pool's
+// pairs and one level below them). Measured (B200, enumeration only, walking
+// every vertex -> this rule): 160 queries of 4-32 vertices on the scale-20
+// graph in one batch 480 -> 80 ms; 16 12-vertex queries one by one 25.1 -> 5.1
+// ms, nine of 24-32 vertices 31.6 -> 3.4 ms. One warp, lane = place in the matching
+// order; returns the place's walked depths before it (home + 1) for a counted
+// place of ord, ~0 otherwise.
+__device__ u32 sink_plan_warp(QState& q, bool may_count) {
+    constexpr float MAX_BITS = 52.f;
+    const QDesc* d = q.desc;
+    const u32 n = q.n_enum;
+    const u32 lane = lane_id();
+    const bool act = lane < n;
+    const u32 u = act ? q.order[lane] : 0u;
+    const u32 lab = act ? d->label[u] : 0xFFFFFFFFu;
+    const u32 adj = act ? d->adj[u] : 0u;
+    u32 nb = 0, same = 0;  // neighbours / equal labels by place in the order
+    for (u32 b = 0; b < n; ++b) {
+        const u32 ub = __shfl_sync(FULL_MASK, u, b), lb = __shfl_sync(FULL_MASK, lab, b);
+        if ((adj >> ub) & 1u) nb |= 1u << b;
+        if (b != lane && lb == lab) same |= 1u << b;
+    }
+    const u32 all = n >= 32 ? ~0u : (1u << n) - 1u;
+    const u32 last = 1u << (n - 1);
+    const float bits = log2f((float)(act ? max(q.cnt[u], 1u) : 1u));
+    u32 E = 0;
+    if (may_count && n >= 5) {
+        float used = __shfl_sync(FULL_MASK, bits, n - 1);
+        const u32 may = __ballot_sync(FULL_MASK, act && lane >= 2 && lane + 1 < n && (nb & (~0u << lane)) == 0);
+        for (u32 m = may; m; m &= m - 1) {
+            const u32 i = __ffs(m) - 1;
+            const u32 si = __shfl_sync(FULL_MASK, same, i);
+            const float bi = __shfl_sync(FULL_MASK, bits, i);
+            if ((si & (E | last)) || used + bi > MAX_BITS || __popc(E) + 4u >= n) continue;
+            E |= 1u << i;
+            used += bi;
+        }
+        while (E) {
+            const u32 end = 31u - __clz(all & ~last & ~E);  // the last walked vertex
+            const u32 bad = __ballot_sync(FULL_MASK, ((E >> lane) & 1u) && (((nb | same) >> end) & 1u));
+            if (!bad) break;
+            E &= ~(1u << (31 - __clz(bad)));  // walked: perhaps the last one then
+        }
+    }
+    const u32 walked = all & ~last & ~E, r = __popc(walked);
+    const u32 below = (1u << lane) - 1u;
+    const bool sink = (E >> lane) & 1u;
+    const u32 place = sink ? r + 1u + __popc(E & below) : (lane + 1 == n ? r : __popc(walked & below));
+    if (act) q.ord[place] = u;
+    // walked depths before a counted vertex, and how many it depends on
+    // (its neighbours, and the vertices of its label: they are excluded)
+    const u32 home = __popc(walked & below);
+    const u32 on = (nb | same) & walked & below;
+    const u32 dep = on ? __popc(walked & ((2u << (31 - __clz(on))) - 1u)) : 0u;
+    u32 beg = r + 1u, inval = 0, hit = 0, home_at = 0xFFFFFFFFu;
+    for (u32 m = E; m; m &= m - 1) {
+        const u32 i = __ffs(m) - 1;
+        const u32 pi = __shfl_sync(FULL_MASK, place, i), hi = __shfl_sync(FULL_MASK, home, i);
+        const u32 di = __shfl_sync(FULL_MASK, dep, i), si = __shfl_sync(FULL_MASK, same, i);
+        if (hi <= lane) ++beg;                // home = hi - 1 < lane
+        if (di > lane) inval |= 1u << pi;     // deepest dependency = di - 1 >= lane
+        // walked depth `lane` is order place w: of the counted vertex's label, after it
+        u32 w = 0xFFFFFFFFu, k = lane;
+        if (lane < r) {
+            u32 mm = walked;
+            for (; k; --k) mm &= mm - 1;
+            w = __ffs(mm) - 1;
+            if (w > i && ((si >> w) & 1u)) hit = pi;
+        }
+        if (lane == pi) home_at = hi;
+    }
+    q.sink_beg[lane] = beg;
+    q.sink_inval[lane] = inval;
+    q.sink_hit[lane] = hit;
+    if (lane == 0) q.walk = r + 1u;
+    __syncwarp();
+    return home_at;
+}
+
 // Backward neighbours by depth (matching/EvaluateQuery.cpp:1594-1625: all
 // earlier neighbours, in query-vertex id order), their table rows, the
 // earlier depths sharing the label (only those can collide on a data
 // vertex), and computeMemoryCostInBytes (BuildTable.cpp:300-326). One warp:
 // lane i handles depth i; all loops are warp-uniform.
-__device__ void enum_plan_warp(const DevGraph& g, QState& q) {
+__device__ void enum_plan_warp(const DevGraph& g, QState& q, bool may_count) {
+    const u32 home = sink_plan_warp(q, may_count);
+    const u32 walk = q.walk;
     const QDesc* d = q.desc;
     const u32 nv = d->n;       // query vertices
     const u32 n = q.n_enum;    // depths (n_enum < nv for a decomposition unit)
     const u32 lane = lane_id();
     const bool act = lane < n;
-    const u32 u = act ? q.order[lane] : 0u;          // vertex at depth lane
+    const u32 u = act ? q.ord[lane] : 0u;             // vertex at depth lane
     const u32 lab = act ? d->label[u] : 0xFFFFFFFFu;  // its label
     u32 depth_of = 0;                                 // depth of vertex `lane` (if ordered)
     for (u32 j = 0; j < n; ++j)
@@ -1042,6 +1135,9 @@ __device__ void enum_plan_warp(const DevGraph& g, QState& q) {
         const u32 lb = __shfl_sync(FULL_MASK, lab, b);
         if (b < lane && lb == lab) same |= 1u << b;
     }
+    // a counted vertex excludes the walked ones before it in the order; those
+    // after it exclude themselves from its count (sink_hit)
+    if (home != 0xFFFFFFFFu) same &= (1u << home) - 1u;
     // prefix-intersection cache plan (the bn rows of this lane's depth are in
     // bn_depth[lane][0, k), written by this lane above)
     u32 cm = 0, crow = 0xFFFFFFFFu, cdep = 0;
@@ -1060,15 +1156,15 @@ __device__ void enum_plan_warp(const DevGraph& g, QState& q) {
     // one shallow row is worth caching only as a bitmap tested against the
     // depth-(d-1) row
     if (__popc(cm) < 2 && !(__popc(cm) == 1 && crow != 0xFFFFFFFFu && bm_ok)) cm = 0;
-    // last-two-depth weight memo (see QState::memo_ok): depth n-1 has a cache
-    // and a row at depth n-2; depth n-2 has rows at depths <= n-4 only, all
+    // last-two-depth weight memo (see QState::memo_ok; n = walk): depth n-1 has a
+    // cache and a row at depth n-2; depth n-2 has rows at depths <= n-4 only, all
     // kept in its cache (even a single one) with a bitmap
-    const u32 last = n >= 3 ? n - 1 : 0u;
+    const u32 last = n >= 3 ? walk - 1 : 0u;
     const u32 cm_l = __shfl_sync(FULL_MASK, cm, last), crow_l = __shfl_sync(FULL_MASK, crow, last);
     const u32 cnt_l = __shfl_sync(FULL_MASK, act ? q.cnt[u] : 0u, last);
     const u32 u_l = __shfl_sync(FULL_MASK, u, last);
     // (the memo's exclusions assume a vertex is never its own neighbour)
-    const bool memo = !g.loops && n >= 3 && lane + 2 == n && crow == 0xFFFFFFFFu && cm_all != 0 && bm_ok &&
+    const bool memo = !g.loops && n >= 3 && lane + 2 == walk && crow == 0xFFFFFFFFu && cm_all != 0 && bm_ok &&
                       cm_l != 0 && crow_l != 0xFFFFFFFFu && cnt_l <= PSM_MEMO_CAP;
     if (memo) cm = cm_all;
     const u32 memo_any = __ballot_sync(FULL_MASK, memo);
@@ -1163,6 +1259,7 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
             q.stop = 0;
             q.overtime = 0;
             q.emit_rows = 0;
+            q.sat = 0;
             q.n_enum = d->n;
             q.table_nnz = 0;
             q.memory_bytes = 0;
@@ -1314,7 +1411,7 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
         TSYNC_B(t);
         return true;
     }
-    if (t.warp() == 0 && !skip && q.adj != nullptr) enum_plan_warp(g, q);
+    if (t.warp() == 0 && !skip && q.adj != nullptr) enum_plan_warp(g, q, q.emit_buf == nullptr);
     TSYNC_B(t);
     return true;
 }
@@ -1590,7 +1687,7 @@ cudaError_t psm_prep_grid_max_blocks(int threads, int* blocks) {
 namespace {
 
 __global__ void unit_plan_kernel(DevGraph g, QState* qs, u32 nq) {
-    if (blockIdx.x < nq && threadIdx.x < 32) enum_plan_warp(g, qs[blockIdx.x]);
+    if (blockIdx.x < nq && threadIdx.x < 32) enum_plan_warp(g, qs[blockIdx.x], false);
 }
 
 __global__ void unit_emit_kernel(QState* qs, u32 nq, u32* const* bufs, const u64* caps) {
@@ -1605,6 +1702,7 @@ __global__ void unit_emit_kernel(QState* qs, u32 nq, u32* const* bufs, const u64
         q.alg_bytes = 0;
         q.stop = 0;
         q.overtime = 0;
+        q.sat = 0;
         q.done_ns = 0;
     }
 }

@@ -167,6 +167,24 @@ struct QState {
     u32 memo_tab;
     u32 loops;              // the data graph has a self loop (DevGraph::loops)
     u32 root_cnt;
+    // Counted vertices (prep.cu sink_plan_warp). A query vertex without later
+    // neighbours in the matching order constrains nothing below it, so the
+    // counting search does not branch on it: it multiplies a weight by the
+    // number of its candidates. The enumerator's depths are the places of
+    // `ord`: the walked vertices in the matching order, the order's last
+    // vertex (place walk - 1), then the counted ones (places walk .. n_enum-1,
+    // in the matching order). All by-depth arrays here are by place in ord;
+    // without counted vertices (and always when embeddings are emitted) ord =
+    // order and walk = n_enum.
+    u32 ord[PSM_MAXQ];
+    u32 walk;
+    // Counted vertices whose place in the order follows walked depth x are
+    // places sink_beg[x] .. sink_beg[x+1]-1; those after the last walked
+    // depth, walk - 2, do not depend on it.
+    u32 sink_beg[PSM_MAXQ];
+    u32 sink_inval[PSM_MAXQ];  // by walked depth x: counted places (bits) that depend on a depth >= x
+    u32 sink_hit[PSM_MAXQ];    // by walked depth: the earlier counted place of the same label (0: none)
+    u32 sat;                   // the count passed 2^64 - 1
     // results
     u64 count;
     u64 cap;                // 0 = none
