@@ -17,7 +17,7 @@
 //    shortest backward-neighbour row (the "driver"), binary-searches it in
 //    the other rows and checks it against same-label earlier vertices; a
 //    ballot compacts the survivors. The last two depths are fused: each lane
-//    takes one candidate of depth n-2 and counts its completions itself;
+//    takes one candidate of the last walked depth and counts its completions;
 //  - query vertices without later neighbours in the matching order are not
 //    branched on: their candidates are counted and multiplied (QState::ord,
 //    weigh_prefix). The depths below are the walked ones;
@@ -153,8 +153,6 @@ struct WarpStack {
     u32 svalid;         // counted places whose candidates (sn) and row bytes (sby) are current
     u32 sn[PSM_MAXQ];
     u64 sby[PSM_MAXQ];
-    u64 late;           // product of the counts after the last walked depth
-    u64 late_by;        // algorithmic bytes of their intersections
     u64 W[PSM_MAXQ];    // by walked depth: product of the counts up to it
     u32 chunk[PSM_MAXQ][32];
 };
@@ -559,9 +557,9 @@ __device__ bool sink_has(const QState& q, u32 s, const WarpStack* ws, u32 v) {
 // less the walked vertices among its candidates. W is also the number of the
 // order's partial embeddings that this prefix stands for, so with `account`
 // the counted vertices' algorithmic bytes are added once per such partial
-// embedding. When the last walked depth comes next, the counted vertices after
-// it (independent of it) are taken too (ws->late, ws->late_by). A count is
-// kept (ws->sn, ws->sby) until a walked depth that it depends on changes.
+// embedding. When the last walked depth comes next, the tail places that do not
+// depend on it are counted too. A count is kept (ws->sn, ws->sby) until a walked
+// depth that it depends on changes.
 // Returns whether the prefix has any completion as far as is known.
 // Warp-uniform; not inlined: a query without counted vertices pays neither
 // registers nor instruction cache for it.
@@ -577,15 +575,11 @@ __device__ __noinline__ bool weigh_prefix(const QState& q, u32 d, WarpStack* ws,
             if (q.sink_hit[j] == h && sink_has(q, h, ws, ws->vid[j])) --now;
         w = w / now * (now - 1u);
     }
-    const u32 e = q.sink_beg[d + 1], end = d + 3 == q.walk ? q.n_enum : e;
-    u64 f = w, by = 0, head = 0, head_by = 0;
-    u32 s = q.sink_beg[d];
-    for (;; ++s) {
-        if (s == e) {  // the rest comes after the last walked depth
-            head = f, head_by = by;
-            f = f ? 1 : 0, by = 0;
-        }
-        if (s >= end || f == 0) break;
+    u64 by = 0;
+    u32 todo = (u32)((1ull << q.sink_beg[d + 1]) - (1ull << q.sink_beg[d]));  // places, as bits
+    if (d + 3 == q.walk) todo |= (((1u << q.tail) - 1u) << (q.walk - 1)) & ~q.lane_tail;
+    for (; todo && w; todo &= todo - 1) {
+        const u32 s = __ffs(todo) - 1;
         if (!((ws->svalid >> s) & 1u)) {
             u64 rows = 0;
             const u32 c = (u32)count_last<IS>(q, s, ws, rows);
@@ -597,19 +591,18 @@ __device__ __noinline__ bool weigh_prefix(const QState& q, u32 d, WarpStack* ws,
             }
             __syncwarp();
         }
-        by += f * ws->sby[s];
-        f *= ws->sn[s];
+        if (s >= q.walk - 1 + q.tail) {
+            by += w * ws->sby[s];
+            w *= ws->sn[s];
+        }
     }
-    if (s < e) head_by = by;  // no candidates: head = 0
     __syncwarp();
     if (lane_id() == 0) {
-        ws->W[d] = head;
-        ws->late = f;
-        ws->late_by = by;
-        if (account) ws->bytes += head_by;
+        ws->W[d] = w;
+        if (account) ws->bytes += by;
     }
     __syncwarp();
-    return head != 0;
+    return w != 0;
 }
 
 // Emits the embeddings of the last depth (original data ids, indexed by
@@ -669,9 +662,9 @@ __device__ u64 emit_last(QState& q, const DevGraph& g, u32 d, WarpStack* ws) {
     return c;
 }
 
-// Last-depth counts of the fused last two depths. The lane's own candidate
-// p (data vertex v) sits at depth dl - 1, the rest of the prefix is shared
-// in ws. A count is the number of positions in the intersection of the
+// Counts of the fused last depths, at place dl of the tail. The lane's own
+// candidate p (data vertex v) sits at the last walked depth dp, the rest of
+// the prefix is shared in ws. A count is the number of positions in the intersection of the
 // backward-neighbour rows of depth dl whose data vertex differs from every
 // same-label vertex of the embedding. With `cached`, depth dl's cache S
 // (warp-shared, valid for the prefix) stands for the rows of depths
@@ -686,10 +679,9 @@ __device__ u64 emit_last(QState& q, const DevGraph& g, u32 d, WarpStack* ws) {
 // ws) whose position lies in S of dl and, when has_row, in R = adj[lo, hi).
 // R is then v's own row, which holds v only through a self loop: without
 // one, v is not looked up.
-__device__ __forceinline__ u32 cached_exclusions(const QState& q, u32 dl, u32 v, const WarpStack* ws, bool has_row,
-                                                 u32 lo, u32 hi) {
+__device__ __forceinline__ u32 cached_exclusions(const QState& q, u32 dl, u32 dp, u32 v, const WarpStack* ws,
+                                                 bool has_row, u32 lo, u32 hi) {
     const u32 u = q.ord[dl];
-    const u32 dp = dl - 1;
     u32 c = 0;
     for (u32 m = q.same_mask[dl]; m; m &= m - 1) {
         const u32 j = __ffs(m) - 1;
@@ -701,10 +693,9 @@ __device__ __forceinline__ u32 cached_exclusions(const QState& q, u32 dl, u32 v,
 }
 
 template <u32 IS>
-__device__ u64 lane_last_count(const QState& q, u32 dl, bool cached, u32 p, u32 v, const WarpStack* ws, u64& bytes,
-                               u64& calls, bool* defer, u32 act) {
+__device__ __forceinline__ u64 lane_last_count(const QState& q, u32 dl, u32 dp, bool cached, u32 p, u32 v,
+                                               const WarpStack* ws, u64& bytes, u64& calls, bool* defer, u32 act) {
     const u32 nb = q.nbn[dl];
-    const u32 dp = dl - 1;
     const u32 long_bm = min(LONG_BM_ROW, DEFER_BM_PER_LANE * act);
     const u32 long_row = min(LONG_ROW, max(2u, DEFER_ROW_PER_LANE * act));
     if (cached) {
@@ -713,7 +704,7 @@ __device__ u64 lane_last_count(const QState& q, u32 dl, bool cached, u32 p, u32 
         bytes += 8ull * nb + 4ull * ws->csum[dl];
         if (k == NO_ROW) {
             calls += s;
-            return s - cached_exclusions(q, dl, v, ws, false, 0, 0);
+            return s - cached_exclusions(q, dl, dp, v, ws, false, 0, 0);
         }
         const u32 base = q.bn_tab[dl][k] + p;
         const u32 lo = q.P[base], hi = q.P[base + 1], r = hi - lo;
@@ -744,7 +735,7 @@ __device__ u64 lane_last_count(const QState& q, u32 dl, bool cached, u32 p, u32 
                 for (u32 i = 0; i < s; ++i) c += contains_u32(q.adj, lo, hi, S[i]);
             }
         }
-        return c - cached_exclusions(q, dl, v, ws, true, lo, hi);
+        return c - cached_exclusions(q, dl, dp, v, ws, true, lo, hi);
     }
     u32 blo = 0, bhi = 0, blen = 0xFFFFFFFFu, bk = 0;
     u64 by = 0;
@@ -807,10 +798,10 @@ __device__ u64 lane_last_count(const QState& q, u32 dl, bool cached, u32 p, u32 
 // against the other arrays. Rows and bytes were counted by the lane that
 // deferred it.
 template <u32 IS>
-__device__ u64 warp_last_count(const QState& q, u32 dl, bool cached, u32 p, u32 v, const WarpStack* ws) {
+__device__ __forceinline__ u64 warp_last_count(const QState& q, u32 dl, u32 dp, bool cached, u32 p, u32 v,
+                                               const WarpStack* ws) {
     const u32 lane = lane_id();
     const u32 nb = q.nbn[dl];
-    const u32 dp = dl - 1;
     if (cached) {
         // deferred only with a row at depth dl - 1
         const u32 s = ws->clen[dl];
@@ -847,7 +838,7 @@ __device__ u64 warp_last_count(const QState& q, u32 dl, bool cached, u32 p, u32 
                 }
             }
         }
-        return c - cached_exclusions(q, dl, v, ws, true, lo, hi);
+        return c - cached_exclusions(q, dl, dp, v, ws, true, lo, hi);
     }
     // the shortest row drives; the second shortest is its merge partner
     u32 blo = 0, bhi = 0, blen = 0xFFFFFFFFu, bk = 0;
@@ -1269,20 +1260,24 @@ __device__ __forceinline__ bool dfs(const DevGraph& g, QState& q, u32 qi, u32 d0
             continue;
         }
         if (!EMIT && d + 2 == n) {
-            // The last two depths fused: each lane takes one driver element
-            // of depth d and counts its completions at depth d + 1 on its own.
+            // The last walked depth and the tail fused: each lane takes one
+            // driver element of depth d and counts the tail on its own.
             if (ws->cur[d] < ws->end[d]) {
                 u64 c = 0;
-                u32 act;  // candidates of depth d in this step
                 if (q.memo_ok && ((ws->lvfull >> d) & 1u) && (ws->flg[d] & LV_CACHED) && ((ws->cbits >> d) & 1u) &&
                     ensure_cache<IS>(q, d + 1, ws)) {
                     // the whole level at once through the weight memo
                     const MemoOut mo = memo_count(q, d, ws);
                     c = mo.count;
-                    act = (u32)mo.calls;
+                    u64 by = mo.bytes;
+                    if (weights)
+                        for (u32 s = n; s < n - 1 + q.tail; ++s) {
+                            by += c * ws->sby[s];
+                            c *= ws->sn[s];
+                        }
                     if (lane == 0) {
                         ws->calls += mo.calls;
-                        ws->bytes += weights ? mo.bytes * ws->W[d - 1] * ws->late : mo.bytes;
+                        ws->bytes += weights ? by * ws->W[d - 1] : by;
                     }
                     __syncwarp();
                     if (lane == 0) ws->cur[d] = ws->end[d];
@@ -1290,27 +1285,41 @@ __device__ __forceinline__ bool dfs(const DevGraph& g, QState& q, u32 qi, u32 d0
                 } else {
                     const u32 cur = ws->cur[d], end = ws->end[d];
                     const u32 idx = cur + lane;
-                    bool defer = false;
                     const u32* list_d = q.list[q.ord[d]];
-                    // the last depth's cache depends on depths <= d - 1 only
-                    const bool cached = ensure_cache<IS>(q, d + 1, ws);
                     const bool valid = idx < end;
                     const u32 p = valid ? (d == 0 ? idx : drv_elem(q, ws, d, idx)) : 0u;
                     const bool ok = d == 0 ? valid : chunk_accept(q, d, p, valid, ws, list_d);
                     const u32 v = ok ? list_d[p] : 0u;
-                    act = __popc(__ballot_sync(FULL_MASK, ok));
                     u64 by = 0;
-                    if (ok) c = lane_last_count<IS>(q, d + 1, cached, p, v, ws, by, calls_l, &defer, act);
-                    bytes_l += weights ? by * (ws->W[d - 1] * ws->late) : by;
-                    c = warp_sum64(c);
-                    // long intersections deferred by their lanes: whole warp each
-                    u32 dm = __ballot_sync(FULL_MASK, defer);
-                    while (dm) {
-                        const u32 src = __ffs(dm) - 1;
-                        dm &= dm - 1;
-                        c += warp_last_count<IS>(q, d + 1, cached, __shfl_sync(FULL_MASK, p, src),
-                                                 __shfl_sync(FULL_MASK, v, src), ws);
+                    c = ok ? 1 : 0;  // partial embeddings below p, down to the place in turn
+                    for (u32 s = n - 1, e = n - 1 + q.tail; s < e; ++s) {
+                        if (!((q.lane_tail >> s) & 1u)) {
+                            by += c * ws->sby[s];
+                            c *= ws->sn[s];
+                            continue;
+                        }
+                        const u32 act = __popc(__ballot_sync(FULL_MASK, c != 0));
+                        if (act == 0) break;
+                        // the place's cache depends on depths <= d - 1 only
+                        const bool cached = ensure_cache<IS>(q, s, ws);
+                        bool defer = false;
+                        u64 x = 0, rows = 0;
+                        if (c) x = lane_last_count<IS>(q, s, d, cached, p, v, ws, rows, calls_l, &defer, act);
+                        // long intersections deferred by their lanes: whole warp each
+                        u32 dm = __ballot_sync(FULL_MASK, defer);
+                        if (dm) iter |= every - 1u;  // a long step: periodic() comes next
+                        while (dm) {
+                            const u32 src = __ffs(dm) - 1;
+                            dm &= dm - 1;
+                            const u64 y = warp_last_count<IS>(q, s, d, cached, __shfl_sync(FULL_MASK, p, src),
+                                                              __shfl_sync(FULL_MASK, v, src), ws);
+                            if (lane == src) x = y;
+                        }
+                        by += c * rows;
+                        c *= x;
                     }
+                    bytes_l += weights && d ? by * ws->W[d - 1] : by;
+                    c = warp_sum64(c);
                     __syncwarp();
                     if (lane == 0) {
                         ws->calls += min(32u, end - cur);
@@ -1318,19 +1327,13 @@ __device__ __forceinline__ bool dfs(const DevGraph& g, QState& q, u32 qi, u32 d0
                     }
                     __syncwarp();
                 }
-                if (weights) {
-                    // each completion stands for W x late embeddings; the vertices
-                    // counted after depth d are read once per candidate of depth d
-                    const u64 w = ws->W[d - 1], wl = w * ws->late, x = c * wl;
-                    if (lane == 0) ws->bytes += act * w * ws->late_by;
-                    count += x;
-                    if (__umul64hi(c, wl) != 0 || count < x) {
-                        if (lane == 0) count_overflow(q);
-                        go = false;
-                        break;
-                    }
-                } else {
-                    count += c;
+                // each completion stands for W embeddings (below 2^64: the plan)
+                if (weights && d) c *= ws->W[d - 1];
+                count += c;
+                if (count < c) {
+                    if (lane == 0) count_overflow(q);
+                    go = false;
+                    break;
                 }
             } else {
                 if (d == d0) break;
@@ -1424,7 +1427,7 @@ __device__ void run_task(const DevGraph& g, QState* qs, const TaskHdr& t, WarpSt
         return;
     }
     // Edge pool: pairs (root r, depth-1 candidate c) taken from the entries
-    // [b, e) of the first table T[u_0][u_1] (queries of four or more vertices);
+    // [b, e) of the first table T[u_0][u_1] (queries of three or more walked depths);
     // the root of an entry is found by walking the table's row offsets.
     const bool edges = t.kind == KIND_EDGES;
     const u32 d0 = edges ? 2u : t.d0;
@@ -1445,7 +1448,7 @@ __device__ void run_task(const DevGraph& g, QState* qs, const TaskHdr& t, WarpSt
         if (lane < d0) ws->vid[lane] = q.list[q.ord[lane]][ws->pos[lane]];
         __syncwarp();
         if (weights)
-            for (u32 d = 1; d + (t.kind == KIND_FULL ? 1u : 0u) < d0; ++d) weigh_prefix<IS>(q, d, ws, false);
+            for (u32 d = 0; d + (t.kind == KIND_FULL ? 1u : 0u) < d0; ++d) weigh_prefix<IS>(q, d, ws, false);
     }
     for (u32 e = t.b; e < end; ++e) {
         bool enter = true;
@@ -1670,7 +1673,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, 3) enum_kernel(DevGraph 
 }
 
 // Single block: per-query initial pools (edges of the first table for
-// queries of four or more vertices, roots otherwise), their prefix in grabs,
+// queries of three or more walked depths, roots otherwise), their prefix in grabs,
 // the per-query task counts and the queue's sequence numbers.
 __global__ void enum_init_kernel(QState* qs, u32 nq, EnumCtl* ctl, Slot* slots, u32* grab_prefix, PoolInfo* pools,
                                  u32* remaining, QDoneRec* done, u32 exit_keep, u32 total_warps, u64 budget_ns,
@@ -1686,8 +1689,7 @@ __global__ void enum_init_kernel(QState* qs, u32 nq, EnumCtl* ctl, Slot* slots, 
             const QState& q = qs[i];
             PoolInfo pi{KIND_RANGE, 0, 1, 0};
             if (q.status == PSM_DEV_OK && !q.stop && q.root_cnt > 0) {
-                const u32 n = q.n_enum;
-                if (n >= 4) {
+                if (q.walk >= 4) {
                     const u32 tb = q.bn_tab[1][0];
                     pi.kind = KIND_EDGES;
                     pi.first = q.P[tb];

@@ -1010,21 +1010,21 @@ __device__ void cfl_order_select(QState& q, const u32* pw) {
 // enumerator's depths. A vertex is counted instead of walked when
 //  - none of its neighbours comes later in the matching order (its candidates
 //    then only multiply the completions; the order's last vertex is always
-//    counted, by the lanes of the fused last two depths, and the first two
-//    stay walked: the initial pool hands them out);
+//    counted; the first two stay walked);
 //  - no other counted vertex has its label (two of one label would exclude
-//    each other; a walked vertex of its label is handled: sink_hit);
-//  - it neither neighbours nor shares the label of the last walked vertex,
-//    whose candidates the lanes try side by side;
+//    each other; walked vertices of its label are handled: the earlier ones
+//    excluded, the later ones through sink_hit);
+//  - it does not share the label of the last walked vertex when it precedes
+//    that one in the order (the lanes try that vertex's candidates side by
+//    side, so a hit would differ from lane to lane);
 //  - the product of the counted vertices' candidate counts stays below 2^52,
-//    so that a weight never overflows.
-// At least three walked depths and the last vertex remain (the initial pool's
-// pairs and one level below them). Measured (B200, enumeration only, walking
-// every vertex -> this rule): 160 queries of 4-32 vertices on the scale-20
-// graph in one batch 480 -> 80 ms; 16 12-vertex queries one by one 25.1 -> 5.1
-// ms, nine of 24-32 vertices 31.6 -> 3.4 ms. One warp, lane = place in the matching
-// order; returns the place's walked depths before it (home + 1) for a counted
-// place of ord, ~0 otherwise.
+//    so that no weight overflows: the vertices of the largest estimated
+//    fan-out |C(u)| x prod_b nnz(b, u) / (|C(b)||C(u)|) are taken first.
+// Measured (B200, enumeration only, walking every vertex -> this rule): 160
+// queries of 4-32 vertices on the scale-20 graph in one batch 480 -> 70 ms; 16
+// 12-vertex queries one by one 25.1 -> 4.9 ms, nine of 24-32 vertices 31.6 ->
+// 3.1 ms. One warp, lane = place in the matching order; returns, for a counted
+// place of ord, the number of walked depths before it (~0 for a walked one).
 __device__ u32 sink_plan_warp(QState& q, bool may_count) {
     constexpr float MAX_BITS = 52.f;
     const QDesc* d = q.desc;
@@ -1034,57 +1034,68 @@ __device__ u32 sink_plan_warp(QState& q, bool may_count) {
     const u32 u = act ? q.order[lane] : 0u;
     const u32 lab = act ? d->label[u] : 0xFFFFFFFFu;
     const u32 adj = act ? d->adj[u] : 0u;
+    const u32 cnt = act ? max(q.cnt[u], 1u) : 1u;
+    const bool plan = may_count && n >= 4 && !q.empty;
     u32 nb = 0, same = 0;  // neighbours / equal labels by place in the order
+    float fan = log2f((float)cnt);
+    const float bits = fan;
     for (u32 b = 0; b < n; ++b) {
         const u32 ub = __shfl_sync(FULL_MASK, u, b), lb = __shfl_sync(FULL_MASK, lab, b);
-        if ((adj >> ub) & 1u) nb |= 1u << b;
+        const u32 cb = __shfl_sync(FULL_MASK, cnt, b);
         if (b != lane && lb == lab) same |= 1u << b;
+        if ((adj >> ub) & 1u) {
+            nb |= 1u << b;
+            if (plan && b < lane) {
+                const u32 tab = table_base(q, ub, u);
+                fan += log2f((float)max(q.P[tab + cb] - q.P[tab], 1u) / ((float)cb * (float)cnt));
+            }
+        }
     }
     const u32 all = n >= 32 ? ~0u : (1u << n) - 1u;
-    const u32 last = 1u << (n - 1);
-    const float bits = log2f((float)(act ? max(q.cnt[u], 1u) : 1u));
-    u32 E = 0;
-    if (may_count && n >= 5) {
+    u32 E = 1u << (n - 1);
+    if (plan) {
         float used = __shfl_sync(FULL_MASK, bits, n - 1);
-        const u32 may = __ballot_sync(FULL_MASK, act && lane >= 2 && lane + 1 < n && (nb & (~0u << lane)) == 0);
-        for (u32 m = may; m; m &= m - 1) {
-            const u32 i = __ffs(m) - 1;
-            const u32 si = __shfl_sync(FULL_MASK, same, i);
+        u32 may = __ballot_sync(FULL_MASK, act && lane >= 2 && lane + 1 < n && (nb & (~0u << lane)) == 0);
+        while (may) {
+            // the remaining vertex of the largest fan-out
+            float f = (may >> lane) & 1u ? fan : -INFINITY;
+            for (u32 o = 16; o; o >>= 1) f = fmaxf(f, __shfl_xor_sync(FULL_MASK, f, o));
+            const u32 i = __ffs(__ballot_sync(FULL_MASK, ((may >> lane) & 1u) && fan == f)) - 1;
+            may &= ~(1u << i);
             const float bi = __shfl_sync(FULL_MASK, bits, i);
-            if ((si & (E | last)) || used + bi > MAX_BITS || __popc(E) + 4u >= n) continue;
+            if ((__shfl_sync(FULL_MASK, same, i) & E) || used + bi > MAX_BITS) continue;
             E |= 1u << i;
             used += bi;
         }
-        while (E) {
-            const u32 end = 31u - __clz(all & ~last & ~E);  // the last walked vertex
-            const u32 bad = __ballot_sync(FULL_MASK, ((E >> lane) & 1u) && (((nb | same) >> end) & 1u));
-            if (!bad) break;
-            E &= ~(1u << (31 - __clz(bad)));  // walked: perhaps the last one then
-        }
+        const u32 end = 31u - __clz(all & ~E);  // the last walked vertex
+        E &= ~__ballot_sync(FULL_MASK, lane < end && ((E >> lane) & 1u) && ((same >> end) & 1u));
     }
-    const u32 walked = all & ~last & ~E, r = __popc(walked);
+    const u32 walked = all & ~E, r = __popc(walked);
     const u32 below = (1u << lane) - 1u;
-    const bool sink = (E >> lane) & 1u;
-    const u32 place = sink ? r + 1u + __popc(E & below) : (lane + 1 == n ? r : __popc(walked & below));
+    const u32 end = walked ? 31u - __clz(walked) : 0u;
+    const u32 tails = n > 1 ? E & (~0u << end) : 0u, inner = E & ~tails, T = __popc(tails);
+    u32 place = __popc(walked & below);
+    if ((tails >> lane) & 1u) place = r + __popc(tails & below);
+    if ((inner >> lane) & 1u) place = r + T + __popc(inner & below);
     if (act) q.ord[place] = u;
     // walked depths before a counted vertex, and how many it depends on
     // (its neighbours, and the vertices of its label: they are excluded)
     const u32 home = __popc(walked & below);
     const u32 on = (nb | same) & walked & below;
     const u32 dep = on ? __popc(walked & ((2u << (31 - __clz(on))) - 1u)) : 0u;
-    u32 beg = r + 1u, inval = 0, hit = 0, home_at = 0xFFFFFFFFu;
+    u32 beg = r + T, inval = 0, hit = 0, home_at = 0xFFFFFFFFu, lanes = 0;
     for (u32 m = E; m; m &= m - 1) {
         const u32 i = __ffs(m) - 1;
         const u32 pi = __shfl_sync(FULL_MASK, place, i), hi = __shfl_sync(FULL_MASK, home, i);
         const u32 di = __shfl_sync(FULL_MASK, dep, i), si = __shfl_sync(FULL_MASK, same, i);
-        if (hi <= lane) ++beg;                // home = hi - 1 < lane
-        if (di > lane) inval |= 1u << pi;     // deepest dependency = di - 1 >= lane
-        // walked depth `lane` is order place w: of the counted vertex's label, after it
-        u32 w = 0xFFFFFFFFu, k = lane;
+        if (((inner >> i) & 1u) && hi <= lane) ++beg;  // between walked depths hi - 1 < lane and hi
+        if (di > lane) inval |= 1u << pi;              // deepest dependency: depth di - 1 >= lane
+        if (((tails >> i) & 1u) && (di == r || r + 1u == n)) lanes |= 1u << pi;
+        // a walked depth `lane` of the counted vertex's label, after it
         if (lane < r) {
             u32 mm = walked;
-            for (; k; --k) mm &= mm - 1;
-            w = __ffs(mm) - 1;
+            for (u32 k = lane; k; --k) mm &= mm - 1;
+            const u32 w = __ffs(mm) - 1;
             if (w > i && ((si >> w) & 1u)) hit = pi;
         }
         if (lane == pi) home_at = hi;
@@ -1092,7 +1103,11 @@ __device__ u32 sink_plan_warp(QState& q, bool may_count) {
     q.sink_beg[lane] = beg;
     q.sink_inval[lane] = inval;
     q.sink_hit[lane] = hit;
-    if (lane == 0) q.walk = r + 1u;
+    if (lane == 0) {
+        q.walk = r + 1u;
+        q.tail = T;
+        q.lane_tail = lanes;
+    }
     __syncwarp();
     return home_at;
 }
@@ -1143,11 +1158,11 @@ __device__ void enum_plan_warp(const DevGraph& g, QState& q, bool may_count) {
     u32 cm = 0, crow = 0xFFFFFFFFu, cdep = 0;
     for (u32 j = 0; j < k; ++j) {
         const u32 bd = q.bn_depth[lane][j];
-        if (bd + 2 <= lane) {
+        if (bd + 2 <= min(lane, walk - 1)) {
             cm |= 1u << j;
             cdep = max(cdep, bd);
         } else {
-            crow = j;  // bd == lane - 1
+            crow = j;  // bd == lane - 1 (the last walked depth for the tail)
         }
     }
     const bool bm_ok = act && q.cnt[u] <= PSM_CACHE_BM_BITS;
@@ -1164,7 +1179,7 @@ __device__ void enum_plan_warp(const DevGraph& g, QState& q, bool may_count) {
     const u32 cnt_l = __shfl_sync(FULL_MASK, act ? q.cnt[u] : 0u, last);
     const u32 u_l = __shfl_sync(FULL_MASK, u, last);
     // (the memo's exclusions assume a vertex is never its own neighbour)
-    const bool memo = !g.loops && n >= 3 && lane + 2 == walk && crow == 0xFFFFFFFFu && cm_all != 0 && bm_ok &&
+    const bool memo = !g.loops && q.lane_tail == 1u << (walk - 1) && n >= 3 && lane + 2 == walk && crow == 0xFFFFFFFFu && cm_all != 0 && bm_ok &&
                       cm_l != 0 && crow_l != 0xFFFFFFFFu && cnt_l <= PSM_MEMO_CAP;
     if (memo) cm = cm_all;
     const u32 memo_any = __ballot_sync(FULL_MASK, memo);

@@ -171,16 +171,18 @@ struct QState {
     // neighbours in the matching order constrains nothing below it, so the
     // counting search does not branch on it: it multiplies a weight by the
     // number of its candidates. The enumerator's depths are the places of
-    // `ord`: the walked vertices in the matching order, the order's last
-    // vertex (place walk - 1), then the counted ones (places walk .. n_enum-1,
-    // in the matching order). All by-depth arrays here are by place in ord;
-    // without counted vertices (and always when embeddings are emitted) ord =
-    // order and walk = n_enum.
+    // `ord`: the walked vertices in the matching order (places 0 .. walk-2),
+    // the counted ones that follow the last walked vertex in the order (`tail`
+    // of them, from place walk - 1), then the other counted ones; both in the
+    // order's sequence. All by-depth arrays here are by place in ord. Without
+    // counted vertices but the order's last one (and always when embeddings
+    // are emitted) ord = order, walk = n_enum and tail = 1.
     u32 ord[PSM_MAXQ];
     u32 walk;
-    // Counted vertices whose place in the order follows walked depth x are
-    // places sink_beg[x] .. sink_beg[x+1]-1; those after the last walked
-    // depth, walk - 2, do not depend on it.
+    u32 tail;
+    u32 lane_tail;             // tail places (bits) that depend on the last walked vertex
+    // Counted vertices whose place in the order lies between walked depths x
+    // and x + 1 are places sink_beg[x] .. sink_beg[x+1]-1.
     u32 sink_beg[PSM_MAXQ];
     u32 sink_inval[PSM_MAXQ];  // by walked depth x: counted places (bits) that depend on a depth >= x
     u32 sink_hit[PSM_MAXQ];    // by walked depth: the earlier counted place of the same label (0: none)
