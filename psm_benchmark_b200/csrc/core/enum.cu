@@ -26,9 +26,10 @@
 //    in chunks by one atomic ticket; queries of up to three vertices hand out
 //    root candidates instead;
 //  - load balance: an idle warp raises a "hungry" counter; while more warps
-//    are hungry than tasks are queued, busy warps donate the upper half of
-//    their shallowest unexplored range (the reference's "linear" split,
-//    TaskPool.cpp:1407-1424) to a bounded lock-free queue;
+//    are hungry than tasks are queued, busy warps donate their shallowest
+//    unexplored range in pieces, but for the first (the reference's "linear"
+//    split, TaskPool.cpp:1407-1424), or the unexplored entries of their
+//    shallowest chunk, up to 32 tasks at a time, to a bounded lock-free queue;
 //  - termination: a pending-work counter (the initial pool + live tasks)
 //    reaches zero. Every wait is bounded by a deadline and an iteration cap;
 //    on expiry the kernel records an error and returns.
@@ -61,25 +62,39 @@ struct Slot {
 
 }  // namespace
 
+// What idle warps poll, read with one 16-byte load.
+struct __align__(16) IdleWords {
+    int avail;          // queued tasks that nobody has claimed (transiently negative)
+    u32 hungry;         // idle warps
+    unsigned long long pending;  // initial pool + live tasks
+};
+
+// Launch-wide scheduler state. Words that many warps poll or update have a
+// 128-byte line per purpose: on one line, every donation queued up behind the
+// polls of thousands of idle warps.
 struct EnumCtl {
     u32 ticket;         // next grab of the initial pool
     u32 total_grabs;
-    u32 hungry;
-    u32 q_head;
-    u32 q_tail;
-    u32 error;
     u32 nq;
-    u32 pad;
-    unsigned long long pending;
+    u32 exit_keep;      // > 0: idle warps beyond this many leave once no work is left
     u64 deadline_ns;
+    u32* remaining;     // per query: grabs + donated tasks not yet finished (kept only with `done`)
+    QDoneRec* done;     // per query completion records (host-mapped) or null
+    u32 pad0[22];
+    IdleWords idle;
+    u32 pad1[28];
+    u32 q_head;         // next task to claim
+    u32 pad2[31];
+    u32 q_tail;         // next slot to fill
+    int q_room;         // slots neither filled nor being read
+    u32 pad3[30];
     u64 donations;
     u64 tasks;
     u64 idle_polls;
-    u32* remaining;     // per query: grabs + donated tasks not yet finished
-    QDoneRec* done;     // per query completion records (host-mapped) or null
-    u32 exit_keep;      // > 0: idle warps beyond this many leave once no work is left
-    u32 pad2;
+    u32 error;
+    u32 pad4[25];
 };
+static_assert(sizeof(EnumCtl) == 5 * 128, "a line per group of words");
 
 namespace {
 
@@ -101,6 +116,15 @@ constexpr u32 BM_WORDS = PSM_CACHE_BM_BITS / 32;
 constexpr u32 SLOT_WORDS = CACHE_CAP + BM_WORDS;
 constexpr u32 WARP_CACHE_WORDS = PSM_MAXQ * SLOT_WORDS + PSM_MEMO_CAP;  // slots + weight memo
 constexpr u32 NO_ROW = 0xFFFFFFFFu;
+// An idle warp polls every IDLE_NS_PER_WARP x (idle warps) ns: 1/2, 1/4 and 1/8
+// of this rate were compared at 3,552 warps, 4 ns (14 us when all are idle,
+// bounded to 8 us) was the fastest. MAX_PIECES: tasks a long range is cut into
+// at a time (1: a 7-vertex query 2.4 ms, 8-32: 1.1 ms). While warps are idle a
+// busy warp looks again after IDLE_STEPS steps (16: 1.1 ms, 4: 0.8 ms).
+constexpr u32 IDLE_NS_PER_WARP = 4;
+constexpr u32 IDLE_NS_MAX = 8000;
+constexpr u32 MAX_PIECES = 16;
+constexpr u32 IDLE_STEPS = 4;
 // Loop steps of a search between two periodic() calls. Where counted vertices
 // multiply, a prefix may stand for 1e6 embeddings, so a capped query's end has
 // to be seen sooner, and a local count of cap / 8192 is published at once: 12-
@@ -1006,85 +1030,54 @@ __device__ __forceinline__ MemoOut memo_count(const QState& q, u32 d, WarpStack*
 
 // ---------------------------------------------------------------- queue --
 
-// Bounded lock-free MPMC ring with a sequence number per slot. Lane 0 claims
-// a slot; the warp copies the task words. A failed claim backs off and gives
-// up after a few tries (the caller keeps the work).
-__device__ bool enqueue(EnumCtl* ctl, Slot* slots, const TaskHdr& h, const WarpStack* ws, u32 npos, u32 extra_at,
-                        u32 extra_val) {
-    const u32 lane = lane_id();
-    u32 slot_idx = 0;
-    int ok = 0;
-    if (lane == 0) {
-        u32 pos = ld_volatile_u32(&ctl->q_tail);
-        for (int it = 0; it < 8; ++it) {
-            Slot* s = slots + (pos % QCAP);
-            u32 seq = ld_acquire_u32(&s->seq);
-            int diff = (int)(seq - pos);
-            if (diff == 0) {
-                u32 prev = atomicCAS(&ctl->q_tail, pos, pos + 1);
-                if (prev == pos) {
-                    ok = 1;
-                    slot_idx = pos;
-                    break;
-                }
-                pos = prev;
-            } else if (diff < 0) {
-                break;  // full
-            } else {
-                pos = ld_volatile_u32(&ctl->q_tail);
-            }
-        }
-    }
-    ok = __shfl_sync(FULL_MASK, ok, 0);
-    if (!ok) return false;
-    slot_idx = __shfl_sync(FULL_MASK, slot_idx, 0);
-    Slot* s = slots + (slot_idx % QCAP);
-    if (lane < HDR_WORDS) {
-        const u32 hv[HDR_WORDS] = {h.kind, h.qi, h.d0, h.b, h.e, h.drv};
-        u32 val = 0;
-#pragma unroll
-        for (u32 i = 0; i < HDR_WORDS; ++i)
-            if (lane == i) val = hv[i];
-        s->w[lane] = val;
-    }
-    s->w[HDR_WORDS + lane] = lane == extra_at ? extra_val : (lane < npos ? ws->pos[lane] : 0u);
-    __threadfence();
-    __syncwarp();
-    if (lane == 0) st_release_u32(&s->seq, slot_idx + 1);
-    return true;
+// A bounded ring of tasks with a sequence number per slot. Producers reserve
+// room and take slots, consumers claim published tasks, each with one fetch-add
+// that always succeeds: with compare-and-swap loops on head and tail the whole
+// launch passed about one task per microsecond from warp to warp while
+// thousands of idle warps retried (a 7-vertex query of 75 M embeddings kept the
+// warps 5 % busy for 8-11 ms; now 60 % for 0.75 ms). A consumer may find that its
+// slot's producer is still writing, and a producer that its slot's last reader
+// is still reading: both are running, so the (bounded) waits are short.
+
+// One poll of the idle words.
+__device__ __forceinline__ IdleWords poll_idle(const EnumCtl* ctl) {
+    ulonglong2 v = make_ulonglong2(0, 0);
+    if (lane_id() == 0) v = __ldcv((const ulonglong2*)&ctl->idle);
+    v.x = __shfl_sync(FULL_MASK, v.x, 0);
+    v.y = __shfl_sync(FULL_MASK, v.y, 0);
+    return IdleWords{(int)(u32)v.x, (u32)(v.x >> 32), v.y};
 }
 
-// Takes a task; its prefix positions go straight into ws->pos.
+// Waits until the slot's sequence number is `want` (lanes with `on`); false
+// after the iteration limit.
+__device__ __forceinline__ bool await_slot(const Slot* s, u32 want, bool on) {
+    for (u32 it = 0; it < (1u << 20); ++it) {
+        const bool ready = !on || ld_acquire_u32(&s->seq) == want;
+        if (__all_sync(FULL_MASK, ready)) return true;
+        __nanosleep(64);
+    }
+    return false;
+}
+
+// Claims a task; its prefix positions go straight into ws->pos.
 __device__ bool dequeue(EnumCtl* ctl, Slot* slots, TaskHdr& h, WarpStack* ws) {
     const u32 lane = lane_id();
-    u32 slot_idx = 0;
-    int ok = 0;
+    u32 at = 0, ok = 0;
     if (lane == 0) {
-        u32 pos = ld_volatile_u32(&ctl->q_head);
-        for (int it = 0; it < 4; ++it) {
-            Slot* s = slots + (pos % QCAP);
-            u32 seq = ld_acquire_u32(&s->seq);
-            int diff = (int)(seq - (pos + 1));
-            if (diff == 0) {
-                u32 prev = atomicCAS(&ctl->q_head, pos, pos + 1);
-                if (prev == pos) {
-                    ok = 1;
-                    slot_idx = pos;
-                    break;
-                }
-                pos = prev;
-                __nanosleep(32u << it);
-            } else if (diff < 0) {
-                break;  // empty
-            } else {
-                pos = ld_volatile_u32(&ctl->q_head);
-            }
+        if (atomicSub(&ctl->idle.avail, 1) > 0) {
+            at = atomicAdd(&ctl->q_head, 1u);
+            ok = 1;
+        } else {
+            atomicAdd(&ctl->idle.avail, 1);
         }
     }
-    ok = __shfl_sync(FULL_MASK, ok, 0);
-    if (!ok) return false;
-    slot_idx = __shfl_sync(FULL_MASK, slot_idx, 0);
-    Slot* s = slots + (slot_idx % QCAP);
+    if (!__shfl_sync(FULL_MASK, ok, 0)) return false;
+    at = __shfl_sync(FULL_MASK, at, 0);
+    Slot* s = slots + (at % QCAP);
+    if (!await_slot(s, at + 1, lane == 0)) {
+        if (lane == 0) atomicExch(&ctl->error, 1u);
+        return false;
+    }
     __threadfence();
     u32 hw = lane < HDR_WORDS ? ld_volatile_u32(&s->w[lane]) : 0u;
     h.kind = __shfl_sync(FULL_MASK, hw, 0);
@@ -1096,91 +1089,92 @@ __device__ bool dequeue(EnumCtl* ctl, Slot* slots, TaskHdr& h, WarpStack* ws) {
     ws->pos[lane] = ld_volatile_u32(&s->w[HDR_WORDS + lane]);
     __threadfence();
     __syncwarp();
-    if (lane == 0) st_release_u32(&s->seq, slot_idx + QCAP);
+    if (lane == 0) {
+        st_release_u32(&s->seq, at + QCAP);
+        atomicAdd(&ctl->q_room, 1);
+    }
     return true;
 }
 
-// Hands the upper half of a range to the queue when more warps are hungry
-// than tasks are queued. Returns true if it donated (the range end moved).
-__device__ bool try_donate_range(EnumCtl* ctl, Slot* slots, u32 kind, u32 qi, u32 d0, u32 cur, u32& end, u32 drv,
-                                 const WarpStack* ws, u32 min_len) {
-    if (end - cur < min_len) return false;
-    const u32 hungry = warp_ld_volatile_u32(&ctl->hungry);
-    if (hungry == 0) return false;
-    const u32 qlen = warp_ld_volatile_u32(&ctl->q_tail) - warp_ld_volatile_u32(&ctl->q_head);
-    if (qlen >= hungry) return false;
+// Queues up to `want` (<= 32) tasks of query qi, one lane writing each; returns
+// how many. KIND_FULL: the last child entries of depth d0 - 1's chunk; KIND_RANGE
+// and KIND_EDGES: the pieces of `piece` elements that end at `end`.
+__device__ u32 donate(EnumCtl* ctl, Slot* slots, u32 kind, u32 qi, u32 d0, u32 end, u32 piece, u32 want,
+                      const WarpStack* ws) {
     const u32 lane = lane_id();
-    const u32 mid = cur + ((end - cur) >> 1);
-    TaskHdr h{kind, qi, d0, mid, end, drv};
+    u32 k = 0, at = 0;
     if (lane == 0) {
-        atomicAdd(&ctl->pending, 1ull);
-        atomicAdd(&ctl->remaining[qi], 1u);
+        const int room = atomicSub(&ctl->q_room, (int)want);
+        k = room <= 0 ? 0u : min((u32)room, want);
+        if (k < want) atomicAdd(&ctl->q_room, (int)(want - k));
+        if (k) {
+            atomicAdd(&ctl->idle.pending, (unsigned long long)k);
+            if (ctl->done) atomicAdd(&ctl->remaining[qi], k);
+            at = atomicAdd(&ctl->q_tail, k);
+            atomicAdd((unsigned long long*)&ctl->donations, (unsigned long long)k);
+        }
+    }
+    k = __shfl_sync(FULL_MASK, k, 0);
+    if (k == 0) return 0;
+    at = __shfl_sync(FULL_MASK, at, 0);
+    Slot* s = slots + ((at + lane) % QCAP);
+    if (!await_slot(s, at + lane, lane < k) && lane == 0) atomicExch(&ctl->error, 1u);
+    if (lane < k) {
+        const bool entry = kind == KIND_FULL;
+        s->w[0] = kind;
+        s->w[1] = qi;
+        s->w[2] = d0;
+        s->w[3] = entry ? 0u : end - (lane + 1) * piece;
+        s->w[4] = entry ? 0u : end - lane * piece;
+        s->w[5] = kind == KIND_RANGE ? ws->drv[d0] | ((u32)ws->flg[d0] << 16) : 0u;  // driver's bn index, level flags
+        for (u32 i = 0; i + (entry ? 1u : 0u) < d0; ++i) s->w[HDR_WORDS + i] = ws->pos[i];
+        if (entry) s->w[HDR_WORDS + d0 - 1] = ws->chunk[d0 - 1][ws->cn[d0 - 1] - 1 - lane];
+        __threadfence();
+        st_release_u32(&s->seq, at + lane + 1);
     }
     __threadfence();
     __syncwarp();
-    if (enqueue(ctl, slots, h, ws, d0, 0xFFFFFFFFu, 0)) {
-        if (lane == 0) atomicAdd((unsigned long long*)&ctl->donations, 1ull);
-        end = mid;
-        return true;
-    }
-    if (lane == 0) {
-        atomicSub(&ctl->remaining[qi], 1u);  // the donor's own task still holds the query open
-        atomicAdd(&ctl->pending, (unsigned long long)-1ll);
-    }
-    return false;
+    if (lane == 0) atomicAdd(&ctl->idle.avail, (int)k);
+    return k;
 }
 
 // Every STEPS warp steps inside a search: donate work to hungry warps, publish
 // the local count (so a capped query stops close to its cap) and stop on the
 // cap or the time limit. Returns true when the search must stop.
-__device__ bool periodic(QState& q, u32 qi, WarpStack* ws, u32 d, u32 d0, u32 iter, u64& count, EnumCtl* ctl,
+__device__ bool periodic(QState& q, u32 qi, WarpStack* ws, u32 d, u32 d0, u32& iter, u64& count, EnumCtl* ctl,
                          Slot* slots) {
     const u32 lane = lane_id();
-    if (warp_ld_volatile_u32(&ctl->hungry) > 0) {
-        // (a) upper half of the shallowest driver range with >= 64 unexplored
-        // elements, else (b) the last unexplored chunk entry of the
-        // shallowest depth below d, as a task one level deeper.
+    const IdleWords idle = poll_idle(ctl);
+    if ((int)idle.hungry > max(idle.avail, 0)) {
+        const u32 room = min(idle.hungry - (u32)max(idle.avail, 0), 32u);
+        // (a) the upper part of the shallowest driver range with >= 64
+        // unexplored elements, else (b) unexplored chunk entries of the
+        // shallowest depth below d, as tasks one level deeper.
         u32 dd = d0;
         for (; dd <= d; ++dd)
             if (ws->end[dd] - ws->cur[dd] >= 64u) break;
         if (dd <= d) {
-            u32 end = ws->end[dd];
-            // drv word: bn index of the driver | level flags << 16
-            bool done = try_donate_range(ctl, slots, KIND_RANGE, qi, dd, ws->cur[dd], end,
-                                         ws->drv[dd] | (ws->flg[dd] << 16), ws, 64u);
+            const u32 len = ws->end[dd] - ws->cur[dd];
+            const u32 parts = min(len / 32u, min(room, MAX_PIECES) + 1u), piece = len / parts;
+            const u32 given = donate(ctl, slots, KIND_RANGE, qi, dd, ws->end[dd], piece, parts - 1u, ws);
             __syncwarp();
-            if (done && lane == 0) {
-                ws->end[dd] = end;
+            if (given && lane == 0) {
+                ws->end[dd] -= given * piece;
                 ws->lvfull &= ~(1u << dd);
             }
-            __syncwarp();
         } else {
             u32 de = d0;
             for (; de < d; ++de)
                 if (ws->cn[de] > ws->ci[de]) break;
-            const u32 hungry = warp_ld_volatile_u32(&ctl->hungry);
-            const u32 qlen = warp_ld_volatile_u32(&ctl->q_tail) - warp_ld_volatile_u32(&ctl->q_head);
-            if (de < d && qlen < hungry) {
-                TaskHdr h{KIND_FULL, qi, de + 1, 0, 0, 0};
-                if (lane == 0) {
-                    atomicAdd(&ctl->pending, 1ull);
-                    atomicAdd(&ctl->remaining[qi], 1u);
-                }
-                __threadfence();
+            if (de < d) {
+                const u32 left = ws->cn[de] - ws->ci[de];
+                const u32 given = donate(ctl, slots, KIND_FULL, qi, de + 1, 0, 0, min(left, room), ws);
                 __syncwarp();
-                if (enqueue(ctl, slots, h, ws, de, de, ws->chunk[de][ws->cn[de] - 1])) {
-                    __syncwarp();
-                    if (lane == 0) {
-                        ws->cn[de] -= 1;
-                        atomicAdd((unsigned long long*)&ctl->donations, 1ull);
-                    }
-                } else if (lane == 0) {
-                    atomicSub(&ctl->remaining[qi], 1u);
-                    atomicAdd(&ctl->pending, (unsigned long long)-1ll);
-                }
-                __syncwarp();
+                if (given && lane == 0) ws->cn[de] -= given;
             }
         }
+        __syncwarp();
+        iter |= (STEPS_WEIGHTED - 1u) & ~(IDLE_STEPS - 1u);
     }
     // Far from the cap a warp publishes every 16 K embeddings. Once its own
     // publish shows the query within reach of the cap (every warp's
@@ -1514,7 +1508,13 @@ __device__ void run_task(const DevGraph& g, QState* qs, const TaskHdr& t, WarpSt
             enter = false;
         }
         if (!dfs<IS, EMIT>(g, q, t.qi, d0, enter, ws, ctl, slots, count, iter)) break;
-        if (edges && e + 2 < end) try_donate_range(ctl, slots, KIND_EDGES, t.qi, 0, e + 1, end, 0, ws, 2u);
+        if (edges && e + 2 < end) {
+            const IdleWords idle = poll_idle(ctl);
+            if ((int)idle.hungry > max(idle.avail, 0)) {
+                const u32 half = (end - e - 1) / 2;
+                end -= half * donate(ctl, slots, KIND_EDGES, t.qi, 0, end, half, 1, ws);
+            }
+        }
     }
     release_caches(q, ws);
     publish(q, count, ws);
@@ -1530,11 +1530,11 @@ __device__ bool take_initial(EnumCtl* ctl, const u32* grab_prefix, const PoolInf
     if (warp_ld_volatile_u32(&ctl->ticket) >= ctl->total_grabs) return false;
     u32 r = 0, crossing = 0;
     if (lane == 0) {
-        atomicAdd(&ctl->pending, 1ull);
+        atomicAdd(&ctl->idle.pending, 1ull);
         __threadfence();
         r = atomicAdd(&ctl->ticket, 1u);
         if (r >= ctl->total_grabs) {
-            atomicAdd(&ctl->pending, (unsigned long long)-1ll);
+            atomicAdd(&ctl->idle.pending, (unsigned long long)-1ll);
         } else if (r + 1 == ctl->total_grabs) {
             crossing = 1;  // this grab exhausts the pool: release the pool's token
         }
@@ -1544,7 +1544,7 @@ __device__ bool take_initial(EnumCtl* ctl, const u32* grab_prefix, const PoolInf
     if (r >= ctl->total_grabs) return false;
     if (crossing && lane == 0) {
         __threadfence();
-        atomicAdd(&ctl->pending, (unsigned long long)-1ll);
+        atomicAdd(&ctl->idle.pending, (unsigned long long)-1ll);
     }
     u32 lo = 0, hi = ctl->nq;  // query owning grab r
     while (hi - lo > 1) {
@@ -1568,10 +1568,10 @@ __device__ bool take_initial(EnumCtl* ctl, const u32* grab_prefix, const PoolInf
             while (cur < end) {
                 const u32 prev = atomicCAS(&ctl->ticket, cur, end);
                 if (prev == cur) {
-                    atomicSub(&ctl->remaining[lo], end - cur);
+                    if (ctl->done) atomicSub(&ctl->remaining[lo], end - cur);
                     if (end == ctl->total_grabs) {
                         __threadfence();
-                        atomicAdd(&ctl->pending, (unsigned long long)-1ll);
+                        atomicAdd(&ctl->idle.pending, (unsigned long long)-1ll);
                     }
                     break;
                 }
@@ -1614,13 +1614,18 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, 3) enum_kernel(DevGraph 
     }
     __syncwarp();
     TaskHdr t;
-    bool hungry = false;
+    bool hungry = false, pool = true;  // pool: the initial pool may have grabs left
     u64 spins = 0, ntasks = 0, npolls = 0;
     while (true) {
-        bool got = take_initial(ctl, grab_prefix, pools, qs, t);
-        if (!got) got = dequeue(ctl, slots, t, ws);
+        bool got = pool && take_initial(ctl, grab_prefix, pools, qs, t);
+        IdleWords idle{};
+        if (!got) {
+            pool = false;  // the ticket never comes back
+            idle = poll_idle(ctl);
+            got = idle.avail > 0 && dequeue(ctl, slots, t, ws);
+        }
         if (got) {
-            if (hungry && lane == 0) atomicSub(&ctl->hungry, 1u);
+            if (hungry && lane == 0) atomicSub(&ctl->idle.hungry, 1u);
             hungry = false;
             spins = 0;
             run_task<IS, EMIT>(g, qs, t, ws, ctl, slots);
@@ -1629,28 +1634,24 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, 3) enum_kernel(DevGraph 
             if (lane == 0) {
                 __threadfence();
                 // the query's last task publishes its result
-                if (atomicSub(&ctl->remaining[t.qi], 1u) == 1u && ctl->done) finish_query(qs[t.qi], ctl->done + t.qi);
-                atomicAdd(&ctl->pending, (unsigned long long)-1ll);
+                if (ctl->done && atomicSub(&ctl->remaining[t.qi], 1u) == 1u) finish_query(qs[t.qi], ctl->done + t.qi);
+                atomicAdd(&ctl->idle.pending, (unsigned long long)-1ll);
             }
             continue;
         }
-        if (!hungry && lane == 0) atomicAdd(&ctl->hungry, 1u);
+        if (!hungry && lane == 0) atomicAdd(&ctl->idle.hungry, 1u);
         hungry = true;
-        unsigned long long pend = 0;
-        if (lane == 0) pend = ld_acquire_u64((const u64*)&ctl->pending);
-        pend = __shfl_sync(FULL_MASK, pend, 0);
-        if (pend == 0) break;
-        if (ctl->exit_keep && warp_ld_volatile_u32(&ctl->ticket) >= ctl->total_grabs &&
-            warp_ld_volatile_u32(&ctl->q_tail) == warp_ld_volatile_u32(&ctl->q_head)) {
+        if (idle.pending == 0) break;
+        if (ctl->exit_keep && idle.avail <= 0) {
             // nothing to take: leave (freeing the SM for other launches)
             // while more than exit_keep warps stay to take donations
             u32 leave = 0;
             if (lane == 0) {
-                const u32 old = atomicSub(&ctl->hungry, 1u);
+                const u32 old = atomicSub(&ctl->idle.hungry, 1u);
                 if (old > ctl->exit_keep)
                     leave = 1;
                 else
-                    atomicAdd(&ctl->hungry, 1u);
+                    atomicAdd(&ctl->idle.hungry, 1u);
             }
             if (__shfl_sync(FULL_MASK, leave, 0)) break;
         }
@@ -1664,7 +1665,10 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, 3) enum_kernel(DevGraph 
             }
             if (__shfl_sync(FULL_MASK, bail, 0)) break;
         }
-        __nanosleep(256);
+        // The more warps are idle, the longer each sleeps: a queued task is
+        // found by one of them after a poll interval / idle warps either way,
+        // and the polls stay few enough for the donors' updates to get through.
+        __nanosleep(min(max(IDLE_NS_PER_WARP * idle.hungry, 128u), IDLE_NS_MAX));
     }
     if (lane == 0) {
         atomicAdd((unsigned long long*)&ctl->tasks, (unsigned long long)ntasks);
@@ -1730,12 +1734,12 @@ __global__ void enum_init_kernel(QState* qs, u32 nq, EnumCtl* ctl, Slot* slots, 
         grab_prefix[nq] = s_carry;
         ctl->total_grabs = s_carry;
         ctl->ticket = 0;
-        ctl->hungry = 0;
         ctl->q_head = 0;
         ctl->q_tail = 0;
+        ctl->q_room = (int)QCAP;
         ctl->error = 0;
         ctl->nq = nq;
-        ctl->pending = s_carry > 0 ? 1ull : 0ull;  // the initial pool's token
+        ctl->idle = IdleWords{0, 0, s_carry > 0 ? 1ull : 0ull};  // pending: the initial pool's token
         ctl->deadline_ns = global_timer_ns() + budget_ns;
         ctl->donations = 0;
         ctl->tasks = 0;
