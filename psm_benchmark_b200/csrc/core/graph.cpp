@@ -41,6 +41,7 @@ void free_graph(psm_graph* g) {
     cudaFree(g->d_nbr);
     cudaFree(g->d_lab_off);
     cudaFree(g->d_orig);
+    cudaFree(g->d_sig);
     delete g;
 }
 
@@ -144,6 +145,19 @@ int psm_graph_build(const uint32_t* off, const uint32_t* nbr, const uint32_t* la
     g->dev.nbr = g->d_nbr;
     g->dev.lab_off = g->d_lab_off;
     g->dev.orig = g->d_orig;
+    // the filters work without signatures, so a full device does not fail here
+    if (V && cudaMalloc((void**)&g->d_sig, sizeof(u64) * (size_t)V) == cudaSuccess) {
+        cudaError_t e = psm_launch_signatures(g->dev, g->d_sig, nullptr);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+        if (e != cudaSuccess) {
+            *err = std::string("signatures: ") + cudaGetErrorString(e);
+            free_graph(g);
+            return PSM_ERR_CUDA;
+        }
+        g->dev.sig = g->d_sig;
+    } else {
+        cudaGetLastError();
+    }
     *out = g;
     return PSM_OK;
 }

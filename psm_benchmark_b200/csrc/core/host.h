@@ -20,6 +20,7 @@ struct psm_graph {
     u32* d_nbr = nullptr;
     u32* d_lab_off = nullptr;
     u32* d_orig = nullptr;
+    u64* d_sig = nullptr;
     DevGraph dev{};
     // For memory estimates: sum of degrees per label, and (when L <=
     // LAB_PAIR_MAX) the number of directed edges per label pair.
@@ -78,6 +79,8 @@ int psm_build_qdesc(const psm_graph& g, const psm_query_desc& q, const psm_optio
 size_t psm_qdesc_bytes(const QDesc& d);
 
 // Kernel launchers (prep.cu, enum.cu).
+// Fills sig[V] with the neighbour-label signatures (DevGraph::sig) of g.
+cudaError_t psm_launch_signatures(const DevGraph& g, u64* sig, cudaStream_t st);
 cudaError_t psm_launch_prep_block(const DevGraph& g, QState* qs, u32 nq, u32* ticket, DevArena* arena, int blocks,
                                   int threads, cudaStream_t st);
 cudaError_t psm_launch_prep_grid(const DevGraph& g, QState* qs, void* barrier, DevArena* arena, u64 budget_ns,

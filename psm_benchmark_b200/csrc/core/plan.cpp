@@ -369,6 +369,16 @@ int psm_build_qdesc(const psm_graph& g, const psm_query_desc& qd, const psm_opti
     std::copy(lab.begin(), lab.end(), d->nlf_lab);
     std::copy(cnt.begin(), cnt.end(), d->nlf_cnt);
     std::copy(grp.begin(), grp.end(), d->nlf_grp);
+    for (u32 it = 0; it < d->n + d->nvirt; ++it) {
+        d->nlf_sig[it] = 0;
+        d->nlf_exact[it] = g.L <= 32;
+        for (u32 k = d->nlf_off[it]; k < d->nlf_off[it + 1]; ++k) {
+            const u32 l = d->nlf_lab[k], need = d->nlf_cnt[k];
+            d->nlf_sig[it] |= 1ull << (l & 31u);
+            if (need >= 2) d->nlf_sig[it] |= 1ull << (32 + (l & 31u));
+            if (need > 2 || l >= g.L) d->nlf_exact[it] = 0;
+        }
+    }
     u32 e = 0;
     for (u32 x = 0; x < n; ++x) {
         d->e_first[x] = e;

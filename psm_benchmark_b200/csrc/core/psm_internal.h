@@ -37,6 +37,9 @@ struct DevGraph {
     const u32* lab_off;  // [L+1] bucket ranges
     const u32* orig;     // [V] internal -> original id
     u32 loops;           // some vertex is its own neighbour (a self loop)
+    // [V] neighbour-label signature: bit l % 32 when some neighbour has label
+    // l, bit 32 + l % 32 when two have the same such label (null: not kept).
+    const u64* sig;
 };
 
 #ifndef PSM_B200_H
@@ -71,6 +74,10 @@ struct QDesc {
     u32 item_label[PSM_MAXQ + PSM_MAXOPT];
     u32 item_deg[PSM_MAXQ + PSM_MAXOPT];
     u32 nlf_off[PSM_MAXQ + PSM_MAXOPT + 1];
+    // signature bits that the item's NLF needs (DevGraph::sig); nlf_exact: they
+    // decide it (one bit per label, no label needed more than twice)
+    u64 nlf_sig[PSM_MAXQ + PSM_MAXOPT];
+    u32 nlf_exact[PSM_MAXQ + PSM_MAXOPT];
     u32 nlf_lab[PSM_MAXNLF];
     u32 nlf_cnt[PSM_MAXNLF];
     u32 nlf_grp[PSM_MAXNLF];    // for real vertices: neighbours carrying nlf_lab (bitmask)
