@@ -83,9 +83,14 @@ __device__ __forceinline__ u32 group_lower_bound(const u32* __restrict__ a, u32 
 }
 
 // label_run for the W-lane group of this lane (v and l group-uniform; a
-// group with !valid gets an empty run). Called by the whole warp.
+// group with !valid gets an empty run). The run's two ends are searched side
+// by side, as in group_lower_bound: one load latency per round for both.
+// Called by the whole warp.
 template <u32 W = 8>
 __device__ __forceinline__ void group_label_run(const DevGraph& g, bool valid, u32 v, u32 l, u32& s, u32& e) {
+    static_assert(W == 4 || W == 8 || W == 32, "group width");
+    constexpr u32 M = W == 32 ? ~0u : (1u << (W & 31u)) - 1u;
+    const u32 lg = lane_id() & (W - 1u), sh = lane_id() & ~(W - 1u);
     u32 lo = 0, hi = 0, k1 = 0, k2 = 0;
     if (valid && l < g.L) {
         lo = g.off[v];
@@ -93,8 +98,28 @@ __device__ __forceinline__ void group_label_run(const DevGraph& g, bool valid, u
         k1 = g.lab_off[l];
         k2 = g.lab_off[l + 1];
     }
-    s = group_lower_bound<W>(g.nbr, lo, hi, k1);
-    e = group_lower_bound<W>(g.nbr, s, hi, k2);
+    u32 lo2 = lo, hi2 = hi;
+    while (__any_sync(FULL_MASK, hi - lo > W || hi2 - lo2 > W)) {
+        const u32 n = hi - lo, n2 = hi2 - lo2;
+        const u32 x = n > W ? __ldg(g.nbr + lo + (u32)((u64)n * (lg + 1u) / (W + 1u))) : 0xFFFFFFFFu;
+        const u32 x2 = n2 > W ? __ldg(g.nbr + lo2 + (u32)((u64)n2 * (lg + 1u) / (W + 1u))) : 0xFFFFFFFFu;
+        const u32 c = __popc((__ballot_sync(FULL_MASK, n > W && x < k1) >> sh) & M);
+        const u32 c2 = __popc((__ballot_sync(FULL_MASK, n2 > W && x2 < k2) >> sh) & M);
+        if (n > W) {
+            const u32 base = lo;
+            lo = c ? base + (u32)((u64)n * c / (W + 1u)) + 1u : base;
+            hi = c < W ? base + (u32)((u64)n * (c + 1u) / (W + 1u)) : hi;
+        }
+        if (n2 > W) {
+            const u32 base = lo2;
+            lo2 = c2 ? base + (u32)((u64)n2 * c2 / (W + 1u)) + 1u : base;
+            hi2 = c2 < W ? base + (u32)((u64)n2 * (c2 + 1u) / (W + 1u)) : hi2;
+        }
+    }
+    const u32 x = lg < hi - lo ? __ldg(g.nbr + lo + lg) : 0xFFFFFFFFu;
+    const u32 x2 = lg < hi2 - lo2 ? __ldg(g.nbr + lo2 + lg) : 0xFFFFFFFFu;
+    s = lo + __popc((__ballot_sync(FULL_MASK, lg < hi - lo && x < k1) >> sh) & M);
+    e = lo2 + __popc((__ballot_sync(FULL_MASK, lg < hi2 - lo2 && x2 < k2) >> sh) & M);
 }
 
 __device__ __forceinline__ bool test_bit(const u32* bm, u32 pos) { return (bm[pos >> 5] >> (pos & 31)) & 1u; }

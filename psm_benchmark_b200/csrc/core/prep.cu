@@ -314,33 +314,51 @@ __device__ __forceinline__ void match_add(u32 m, u32& matched, u32& rm) {
 // label, so each neighbour label is matched on its own; right vertices are
 // streamed through an incremental maximum matching (warp-wide).
 __device__ bool gql_check(const DevGraph& g, const QDesc* d, const QState& q, u32 u, u32 v) {
+    // Entries are taken ROW at a time, their loads (and those of their candidate
+    // bits) in flight together. Rows of up to ROW entries are read once, before
+    // the labels are looked at; a label's run is then a compare per entry, and
+    // of a longer row found by the whole warp in two or three loads. With one
+    // search per lane and end (20 dependent loads a label on hub rows) the
+    // refinement steps of an 8-vertex query on the scale-17 graph took 230 us in
+    // all, now 140 us.
+    constexpr u32 PARTS = 4, ROW = 32 * PARTS;
     const u32 lane = lane_id();
-    u32 lo = g.off[v], hi = g.off[v + 1];
+    const u32 lo = g.off[v], hi = g.off[v + 1];
+    const bool held = hi - lo <= ROW;
+    u32 row[PARTS];
+    auto load = [&](u32 from, u32 to) {
+#pragma unroll
+        for (u32 i = 0; i < PARTS; ++i) {
+            const u32 o = from + 32u * i + lane;
+            row[i] = o < to ? __ldg(g.nbr + o) : 0xFFFFFFFFu;  // lies in no bucket
+        }
+    };
+    if (held) load(lo, hi);
     for (u32 k = d->nlf_off[u]; k < d->nlf_off[u + 1]; ++k) {
         const u32 l = d->nlf_lab[k], S = d->nlf_grp[k];
         if (l >= g.L) return false;
-        u32 s = lower_bound_u32(g.nbr, lo, hi, g.lab_off[l]);
-        u32 e = lower_bound_u32(g.nbr, s, hi, g.lab_off[l + 1]);
-        lo = e;
-        const u32 base = g.lab_off[l];
+        const u32 base = g.lab_off[l], top = g.lab_off[l + 1];
         u32 matched = 0, rm = 0;
-        for (u32 j = s; j < e && matched != S; j += 32) {
-            u32 idx = j + lane, m = 0;
-            if (idx < e) {
-                u32 pos = __ldg(g.nbr + idx) - base;
-                u32 x = S;
-                while (x) {
-                    u32 y = __ffs(x) - 1;
-                    x &= x - 1;
-                    if (test_bit(q.bm[y], pos)) m |= 1u << y;
-                }
+        u32 s = lo, e = hi;
+        if (!held) group_label_run<32>(g, true, v, l, s, e);
+        for (u32 j = s; j < e && matched != S; j += ROW) {
+            if (!held) load(j, e);
+            u32 m[PARTS] = {};  // the query vertices that the entry is a candidate of
+            for (u32 x = S; x; x &= x - 1) {
+                const u32 y = __ffs(x) - 1;
+                const u32* bm = q.bm[y];
+#pragma unroll
+                for (u32 i = 0; i < PARTS; ++i)
+                    if (row[i] >= base && row[i] < top && test_bit(bm, row[i] - base)) m[i] |= 1u << y;
             }
-            u32 nz = __ballot_sync(FULL_MASK, m != 0);
-            while (nz && matched != S) {
-                u32 src = __ffs(nz) - 1;
-                nz &= nz - 1;
-                u32 mm = __shfl_sync(FULL_MASK, m, src);
-                match_add(mm, matched, rm);
+#pragma unroll
+            for (u32 i = 0; i < PARTS; ++i) {
+                u32 nz = __ballot_sync(FULL_MASK, m[i] != 0);
+                while (nz && matched != S) {
+                    const u32 src = __ffs(nz) - 1;
+                    nz &= nz - 1;
+                    match_add(__shfl_sync(FULL_MASK, m[i], src), matched, rm);
+                }
             }
         }
         if (matched != S) return false;
@@ -1276,8 +1294,8 @@ __device__ void enum_plan_warp(const DevGraph& g, QState& q, bool may_count) {
 // The preparation of a query is a fixed list of steps, each ending with a
 // team barrier:
 //   0 clear, 1 NLF, 2 pick start vertices,
-//   GQL / NLF filter: compact every u, empty check, [GQL: refine (round, u)
-//     for 2n steps, compact every u],
+//   GQL / NLF filter: compact all, empty check, [GQL: refine (round, u)
+//     for 2n steps, compact all],
 //   CFL filter: compact the start vertex, the plan's generate / prune steps,
 //   then: empty check, tables, order, enumeration plan.
 // run_step executes one step with any team; the drivers below choose teams.
@@ -1292,7 +1310,7 @@ __device__ u32 step_count(const QState& q) {
     if (is_cfl(d))
         mid = 1 + d->fplan[q.froot].nsteps;
     else
-        mid = n + 1 + (d->filter == PSM_FILTER_GQL ? 3 * n : 0);
+        mid = 2 + (d->filter == PSM_FILTER_GQL ? 2 * n + 1 : 0);
     return 3 + mid + 4;
 }
 
@@ -1301,16 +1319,17 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
     const QDesc* d = q.desc;
     const u32 n = d->n;
     const bool cfl = is_cfl(d);
-    if (k == 0) {  // clear bitmaps and counters
-        for (u32 u = 0; u < n; ++u)
-            for (u32 i = t.rank(); i < q.bwords[u]; i += t.size()) q.bm[u][i] = 0;
+    if (k == 0) {
+        // Clear accumulators and counters. Every word of a candidate bitmap is
+        // written (NLF stage, generate steps) before it is read, and the host
+        // hands over zero item counts, so the NLF stage depends on nothing here
+        // and needs no barrier before it (4-8 us of a preparation).
         if (cfl)
             for (u32 i = t.rank(); i < q.acc_words; i += t.size()) {
                 q.acc[i] = 0;
                 q.tmp[i] = 0;
             }
         if (t.rank() == 0) {
-            for (u32 i = 0; i < PSM_MAXQ + PSM_MAXOPT; ++i) q.item_cnt[i] = 0;
             q.empty = 0;
             q.filter_ok = 1;
             q.count = 0;
@@ -1326,7 +1345,6 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
             q.root_cnt = 0;
             q.status = PSM_DEV_OK;
         }
-        TSYNC_B(t);
         return true;
     }
     if (k == 1) {  // NLF candidates of the needed items
@@ -1375,12 +1393,13 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
     }
     u32 j = k - 3;
     if (!cfl) {
-        if (j < n) {  // compact u (NLF result)
-            if (!compact_vertex(t, g, q, j)) return false;
+        const u32 every = n >= 32 ? ~0u : (1u << n) - 1u;
+        if (j == 0) {  // compact every vertex (NLF result), one barrier for all
+            if (!multi_compact(t, g, q, every)) return false;
             TSYNC_B(t);
             return true;
         }
-        j -= n;
+        j -= 1;
         if (j == 0) {  // NLFFilter / GQLFilter stop at the first empty set
             if (t.rank() == 0) {
                 for (u32 u = 0; u < n; ++u)
@@ -1413,12 +1432,12 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
                 return true;
             }
             j -= 2 * n;
-            if (j < n) {
-                if (!q.empty && !compact_vertex(t, g, q, j)) return false;
+            if (j == 0) {
+                if (!q.empty && !multi_compact(t, g, q, every)) return false;
                 TSYNC_B(t);
                 return true;
             }
-            j -= n;
+            j -= 1;
         }
     } else {
         const FilterPlan& fp = d->fplan[q.froot];
@@ -1494,15 +1513,17 @@ __device__ bool step_small(const DevGraph& g, const QState& q, u32 k) {
     }
     u32 j = k - 3;
     if (!is_cfl(d)) {
-        if (j < n) return q.bwords[j] <= SMALL_WORDS;
-        j -= n;
+        u32 words = 0;
+        for (u32 u = 0; u < n; ++u) words += q.bwords[u];
+        if (j == 0) return words <= SMALL_WORDS;
+        j -= 1;
         if (j == 0) return true;
         j -= 1;
         if (d->filter == PSM_FILTER_GQL) {
             if (j < 2 * n) return q.cnt[j % n] <= SMALL_ITEMS / 8;
             j -= 2 * n;
-            if (j < n) return q.bwords[j] <= SMALL_WORDS;
-            j -= n;
+            if (j == 0) return words <= SMALL_WORDS;
+            j -= 1;
         }
     } else {
         const FilterPlan& fp = d->fplan[q.froot];
