@@ -909,10 +909,36 @@ __device__ void estimate_path_block(QState& q, const u32* path, u32 k, u64* est,
         const u32 a = path[i - 1], b = path[i];
         const u32 rb = table_base(q, a, b), rows = q.cnt[a];
         u64 s = 0;
-        for (u32 j = threadIdx.x; j < rows; j += blockDim.x) {
+        for (u32 j0 = threadIdx.x & ~31u; j0 < rows; j0 += blockDim.x) {
+            const u32 j = j0 + lane_id();
+            u32 lo = 0, hi = 0;
+            if (j < rows) {
+                lo = q.P[rb + j];
+                hi = q.P[rb + j + 1];
+            }
+            // a lane sums a short row (four gathers in flight), the warp a long
+            // one: a hub row of a thousand entries on one lane set the time of
+            // a path's level
+            constexpr u32 SHORT = 64;
             u64 ls = 0;
-            for (u32 e = q.P[rb + j]; e < q.P[rb + j + 1]; ++e) ls += child[q.adj[e]];
-            par[j] = ls;
+            if (hi - lo <= SHORT) {
+                u32 e = lo;
+                for (; e + 4u <= hi; e += 4u) {
+                    const u32 a0 = q.adj[e], a1 = q.adj[e + 1], a2 = q.adj[e + 2], a3 = q.adj[e + 3];
+                    const u64 c0 = child[a0], c1 = child[a1], c2 = child[a2], c3 = child[a3];
+                    ls += c0 + c1 + c2 + c3;
+                }
+                for (; e < hi; ++e) ls += child[q.adj[e]];
+            }
+            for (u32 m = __ballot_sync(FULL_MASK, hi - lo > SHORT); m; m &= m - 1) {
+                const u32 src = __ffs(m) - 1;
+                const u32 b = __shfl_sync(FULL_MASK, lo, src), e = __shfl_sync(FULL_MASK, hi, src);
+                u64 x = 0;
+                for (u32 i = b + lane_id(); i < e; i += 32) x += child[q.adj[i]];
+                x = warp_sum64(x);
+                if (lane_id() == src) ls = x;
+            }
+            if (j < rows) par[j] = ls;
             s += ls;
         }
         s = warp_sum64(s);
@@ -928,6 +954,7 @@ __device__ void estimate_path_block(QState& q, const u32* path, u32 k, u64* est,
 // est_out[path_off[p] - p + k] (a path of length l has l - 1 estimates).
 // Paths are independent: with several blocks each block takes its own paths
 // (its own child / parent buffers), so the whole step costs one team barrier.
+// est_out is zeroed at the start of the preparation.
 template <class Team>
 __device__ bool cfl_estimates(Team& t, QState& q, const u32* pw) {
     const QDesc* d = q.desc;
@@ -938,8 +965,6 @@ __device__ bool cfl_estimates(Team& t, QState& q, const u32* pw) {
     const u32 npaths = gfirst[ngroups + 1];
     const u32* poff = gfirst + ngroups + 2;
     const u32* pv = poff + npaths + 1 + ncore;
-    for (u32 i = t.rank(); i < PSM_PLAN_WORDS; i += t.size()) q.est_out[i] = 0;
-    TSYNC_B(t);
     const u32 eb = min(t.nblocks(), q.est_blocks);
     if (t.block() < eb) {
         u64* child = q.est_a + (size_t)t.block() * 2 * q.est_stride;
@@ -951,12 +976,34 @@ __device__ bool cfl_estimates(Team& t, QState& q, const u32* pw) {
     return true;
 }
 
+// Index of the alive entry (bit i of `alive`, 64 at most) with the smallest
+// value(i), the first one on ties and when no value is below the largest
+// double (the reference's strict "<"). A lane evaluates entries lane, lane + 32.
+template <class F>
+__device__ __forceinline__ u32 pick_smallest(u64 alive, F value) {
+    double best = 1.79769313486231570815e308;
+    u32 at = 64;
+    for (u32 i = lane_id(); i < 64; i += 32) {
+        if (!((alive >> i) & 1ull)) continue;
+        const double v = value(i);
+        if (v < best) best = v, at = i;
+    }
+    for (u32 o = 16; o; o >>= 1) {
+        const double v = __shfl_xor_sync(FULL_MASK, best, o);
+        const u32 i = __shfl_xor_sync(FULL_MASK, at, o);
+        if (v < best || (v == best && i < at)) best = v, at = i;
+    }
+    return at < 64 ? at : (u32)__ffsll((long long)alive) - 1u;
+}
+
 // matching/GenerateQueryPlan.cpp:270-471 generateCFLQueryPlan greedy
-// selection (core paths, tree paths per forest, leaves), one thread. Ties
-// keep the first minimum, as the reference's strict "<" does.
+// selection (core paths, tree paths per forest, leaves). One warp: the lanes
+// price the remaining paths side by side. On one thread, every selection walked
+// every X
+// now 126 us.
 __device__ void cfl_order_select(QState& q, const u32* pw) {
     const QDesc* d = q.desc;
-    const u32 n = d->n;
+    const u32 n = d->n, lane = lane_id();
     const u32 root = pw[0];
     const u32* parent = pw + 1;
     const u32 ncore = pw[1 + 2 * n];
@@ -968,105 +1015,57 @@ __device__ void cfl_order_select(QState& q, const u32* pw) {
     const u32* pv = nte + ncore;
     const u32 nleaves = pv[poff[npaths]];
     const u32* leaves = pv + poff[npaths] + 1;
-    const double DMAX = 1.79769313486231570815e308;
     auto est = [&](u32 p, u32 k) { return q.est_out[poff[p] - p + k]; };
     auto path_v = [&](u32 p, u32 k) { return pv[poff[p] + k]; };
     auto plen = [&](u32 p) { return poff[p + 1] - poff[p]; };
-    u32 vis = 1u << root;
-    u32 cnt = 0;
-    q.order[cnt] = root;
-    q.pivot[cnt] = 0;
-    ++cnt;
-    u64 alive = 0;  // remaining paths of the current family (bitmask over <= 64)
+    auto first = [](u32 k) { return k >= 64 ? ~0ull : (1ull << k) - 1ull; };
+    u32 vis = 0, cnt = 0;
+    auto place = [&](u32 x, u32 pivot) {
+        if (lane == 0 && cnt < PSM_MAXQ) {
+            q.order[cnt] = x;
+            q.pivot[cnt] = pivot;
+        }
+        ++cnt;
+        vis |= 1u << x;
+    };
+    // estimate of path p below its last placed vertex, per candidate of it
+    auto price = [&](u32 p) {
+        u32 ri = 0;
+        for (u32 j = 0; j < plen(p); ++j) {
+            if ((vis >> path_v(p, j)) & 1u) continue;
+            ri = j == 0 ? 0u : j - 1u;
+            break;
+        }
+        return (double)est(p, ri) / (double)q.cnt[path_v(p, ri)];
+    };
+    place(root, 0);
     if (ncore > 0) {
-        double mn = DMAX;
-        u32 sel = 0;
-        for (u32 i = 0; i < ncore; ++i) {
-            double v = (double)est(i, 0) / (double)nte[i];
-            if (v < mn) mn = v, sel = i;
-        }
-        for (u32 k = 1; k < plen(sel); ++k) {
-            q.order[cnt] = path_v(sel, k);
-            q.pivot[cnt] = path_v(sel, k - 1);
-            ++cnt;
-            vis |= 1u << path_v(sel, k);
-        }
-        alive = (ncore >= 64 ? ~0ull : ((1ull << ncore) - 1)) & ~(1ull << sel);
-        while (alive) {
-            mn = DMAX;
-            sel = 0xFFFFFFFFu;
-            for (u32 i = 0; i < ncore; ++i) {
-                if (!((alive >> i) & 1ull)) continue;
-                if (sel == 0xFFFFFFFFu) sel = i;  // reference starts from index 0 of the remaining list
-                u32 ri = 0;
-                for (u32 j = 0; j < plen(i); ++j) {
-                    if ((vis >> path_v(i, j)) & 1u) continue;
-                    ri = j - 1;
-                    break;
-                }
-                double v = (double)est(i, ri) / (double)q.cnt[path_v(i, ri)];
-                if (v < mn) mn = v, sel = i;
-            }
-            for (u32 k = 1; k < plen(sel); ++k) {
-                u32 x = path_v(sel, k);
-                if ((vis >> x) & 1u) continue;
-                q.order[cnt] = x;
-                q.pivot[cnt] = path_v(sel, k - 1);
-                ++cnt;
-                vis |= 1u << x;
-            }
-            alive &= ~(1ull << sel);
+        u32 sel = pick_smallest(first(ncore), [&](u32 i) { return (double)est(i, 0) / (double)nte[i]; });
+        for (u32 k = 1; k < plen(sel); ++k) place(path_v(sel, k), path_v(sel, k - 1));
+        for (u64 alive = first(ncore) & ~(1ull << sel); alive; alive &= ~(1ull << sel)) {
+            sel = pick_smallest(alive, price);
+            for (u32 k = 1; k < plen(sel); ++k)
+                if (!((vis >> path_v(sel, k)) & 1u)) place(path_v(sel, k), path_v(sel, k - 1));
         }
     }
     for (u32 gi = 0; gi < ngroups; ++gi) {
         const u32 p0 = gfirst[gi], p1 = gfirst[gi + 1];
-        alive = (p1 - p0 >= 64) ? ~0ull : ((1ull << (p1 - p0)) - 1);
-        while (alive) {
-            double mn = DMAX;
-            u32 sel = 0xFFFFFFFFu;
-            for (u32 i = p0; i < p1; ++i) {
-                if (!((alive >> (i - p0)) & 1ull)) continue;
-                if (sel == 0xFFFFFFFFu) sel = i;
-                u32 ri = 0;
-                for (u32 j = 0; j < plen(i); ++j) {
-                    if ((vis >> path_v(i, j)) & 1u) continue;
-                    ri = j == 0 ? j : j - 1;
-                    break;
-                }
-                double v = (double)est(i, ri) / (double)q.cnt[path_v(i, ri)];
-                if (v < mn) mn = v, sel = i;
-            }
-            for (u32 k = 0; k < plen(sel); ++k) {
-                u32 x = path_v(sel, k);
-                if ((vis >> x) & 1u) continue;
-                q.order[cnt] = x;
-                q.pivot[cnt] = k ? path_v(sel, k - 1) : 0;
-                ++cnt;
-                vis |= 1u << x;
-            }
-            alive &= ~(1ull << (sel - p0));
+        u32 sel = 0;
+        for (u64 alive = first(p1 - p0); alive; alive &= ~(1ull << sel)) {
+            sel = pick_smallest(alive, [&](u32 i) { return price(p0 + i); });
+            const u32 p = p0 + sel;
+            for (u32 k = 0; k < plen(p); ++k)
+                if (!((vis >> path_v(p, k)) & 1u)) place(path_v(p, k), k ? path_v(p, k - 1) : 0u);
         }
     }
-    u32 lalive = nleaves >= 32 ? ~0u : ((1u << nleaves) - 1u);
-    while (lalive) {
-        double mn = DMAX;
-        u32 sel = 0xFFFFFFFFu;
-        for (u32 i = 0; i < nleaves; ++i) {
-            if (!((lalive >> i) & 1u)) continue;
-            if (sel == 0xFFFFFFFFu) sel = i;
-            double v = (double)q.cnt[leaves[i]];
-            if (v < mn) mn = v, sel = i;
-        }
-        u32 l = leaves[sel];
-        if (!((vis >> l) & 1u)) {
-            q.order[cnt] = l;
-            q.pivot[cnt] = parent[l];
-            ++cnt;
-            vis |= 1u << l;
-        }
-        lalive &= ~(1u << sel);
+    u32 sel = 0;
+    for (u64 alive = first(nleaves); alive; alive &= ~(1ull << sel)) {
+        sel = pick_smallest(alive, [&](u32 i) { return (double)q.cnt[leaves[i]]; });
+        const u32 l = leaves[sel];
+        if (!((vis >> l) & 1u)) place(l, parent[l]);
     }
-    if (cnt != n) q.status = PSM_DEV_INTERNAL;
+    if (cnt != n && lane == 0) q.status = PSM_DEV_INTERNAL;
+    __syncwarp();
 }
 
 // Chooses the counted vertices of a query (QState::ord) and orders the
@@ -1329,6 +1328,8 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
                 q.acc[i] = 0;
                 q.tmp[i] = 0;
             }
+        if (d->order == PSM_ORDER_CFL)
+            for (u32 i = t.rank(); i < PSM_PLAN_WORDS; i += t.size()) q.est_out[i] = 0;
         if (t.rank() == 0) {
             q.empty = 0;
             q.filter_ok = 1;
@@ -1481,17 +1482,15 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
             if (d->order == PSM_ORDER_CFL) {
                 const u32* pw = d->plan_words + d->oplan_off[q.oroot];
                 if (!cfl_estimates(t, q, pw)) return false;
-                TSYNC_B(t);
-                if (t.rank() == 0) cfl_order_select(q, pw);
+                if (t.warp() == 0) cfl_order_select(q, pw);
             } else if (t.rank() == 0) {
                 gql_order(g, q);
             }
         }
-        TSYNC_B(t);
-        return true;
+        return true;  // the next step runs on the same warp
     }
+    __syncwarp();
     if (t.warp() == 0 && !skip && q.adj != nullptr) enum_plan_warp(g, q, q.emit_buf == nullptr);
-    TSYNC_B(t);
     return true;
 }
 
