@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -165,6 +166,7 @@ int setup_query(psm_context* ctx, const psm_graph& g, const QDesc& d, const psm_
     q.tmp = b.take<u32>(maxw);
     q.acc_words = maxw;
     q.P = b.take<u32>(rows + 1);
+    q.P_rows = (u32)rows;
     q.scan = b.take<u32>((size_t)scan_words * std::max(d.n, 1u));  // multi_compact: a block's word per vertex
     if (d.order == PSM_ORDER_CFL) {
         // one buffer pair per block that estimates paths concurrently
@@ -192,10 +194,20 @@ int setup_query(psm_context* ctx, const psm_graph& g, const QDesc& d, const psm_
     return PSM_OK;
 }
 
-bool use_cluster_batch(const psm_context* ctx, u32 nq) {
+// Whether a batch of nq queries is prepared with a cluster per query. positions:
+// label-bucket sizes summed over a query's vertices, a batch's mean (0: not
+// known). Clusters spread a query over 8 SMs but run few at a time: their time
+// is nq times a slope, a block's nearly flat until every SM has several. Both
+// measured on R-MAT graphs (B200, 37 clusters), the lines cross at
+//   positions      3,155   12,352   30,822   73,772   605,953
+//   queries           30       55       88      125       270
+// (at 160 queries: 1.03 against 0.20 ms with 3,155 positions, 14.7 against 20.8
+// ms with 605,953), which 30 (positions / 3,200)^0.42 follows.
+bool use_cluster_batch(const psm_context* ctx, u32 nq, double positions) {
     if (ctx->batch_cluster <= 0 || ctx->tune_team == PSM_TEAM_BLOCK) return false;
     if (ctx->tune_team == PSM_TEAM_CLUSTER) return true;
-    return nq <= 4u * (u32)ctx->batch_clusters;
+    if (positions <= 0) return nq <= 4u * (u32)ctx->batch_clusters;
+    return nq <= 30.0 * std::pow(positions / 3200.0, 0.42) * ctx->batch_clusters / 37.0;
 }
 
 // Enumeration grid of a batched launch (the tuning's share of the co-resident blocks).
@@ -246,7 +258,7 @@ char* staging(psm_context* ctx, size_t bytes) {
 // (plain path); otherwise one block per query (batched path).
 int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, u32 nq, const psm_options& opt,
                 bool grid_team, psm_result* results, psm_run* keep, bool prep_only = false, QDoneRec* done = nullptr,
-                u32 exit_keep = 0, void (*poll)(void*) = nullptr, void* poll_arg = nullptr) {
+                u32 exit_keep = 0, void (*poll)(void*) = nullptr, void* poll_arg = nullptr, bool block_team = false) {
     if (!ctx || !g || !qs || nq == 0) return fail(PSM_ERR_ARG, "null argument");
     if (ctx->run_live) return fail(PSM_ERR_ARG, "a psm_run is still alive on this context");
     CK(cudaSetDevice(ctx->device));
@@ -264,21 +276,34 @@ int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, 
     lay.d_enum_q = b.take<char>(psm_enum_query_bytes(nq));
     lay.d_res = b.take<DevResult>(nq);
     if (!lay.d_desc || !lay.d_q || !lay.d_enum_q || !lay.d_res) return fail(PSM_ERR_OOM, "device arena exhausted");
-    // Batched preparation team: a cluster per query while the batch is small
-    // (latency: a query's preparation spreads over the cluster's SMs), a
-    // block per query for large batches (throughput).
-    const bool cluster_batch = !grid_team && use_cluster_batch(ctx, nq);
+    // Batched preparation team: a cluster per query while the batch is small for
+    // its graph (latency: a query's preparation spreads over the cluster's SMs),
+    // a block per query for large batches (throughput).
+    double positions = 0;
+    if (!poll)
+        for (u32 i = 0; i < nq; ++i)
+            for (u32 u = 0; u < descs[i].n; ++u) positions += (double)g->freq(descs[i].label[u]) / nq;
+    const bool cluster_batch = !grid_team && !block_team && use_cluster_batch(ctx, nq, positions);
+    // A cluster keeps path-estimate buffers per block of it: a batch too large
+    // for the arena that way is prepared with a block per query. (A server's
+    // lanes size their batches for the team themselves.)
+    const bool may_shrink = cluster_batch && !poll && ctx->tune_team == PSM_TEAM_RULE;
+    auto with_blocks = [&]() {
+        return run_queries(ctx, g, qs, nq, opt, false, results, keep, prep_only, done, exit_keep, poll, poll_arg, true);
+    };
     // team scans need one word per block of the preparing team (+1)
     const u32 scan_words = grid_team ? (u32)std::max(ctx->prep_grid_blocks, ctx->cluster_size) + 1
                                      : (cluster_batch ? (u32)ctx->batch_cluster : 1u) + 1;
     std::vector<QState> hq(nq);
     for (u32 i = 0; i < nq; ++i) {
         int rc = setup_query(ctx, *g, descs[i], opt, b, lay.d_desc + i, scan_words, hq[i]);
+        if (rc == PSM_ERR_OOM && may_shrink) return with_blocks();
         if (rc) return rc;
     }
     // the rest of the arena is the device-side allocator region (tables)
     DevArena da{};
     size_t start = align_up(b.top);
+    if (start + 4096 > b.cap && may_shrink) return with_blocks();
     if (start + 4096 > b.cap) return fail(PSM_ERR_OOM, "device arena exhausted (no table space)");
     da.base = (u32*)(ctx->arena + start);
     da.top = 0;
@@ -414,6 +439,7 @@ int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, 
         ctx->run_live = true;
     }
     if (worst == PSM_ERR_INTERNAL) return fail(worst, enum_err ? "enumeration wait gave up" : "device error");
+    if (worst == PSM_ERR_OOM && may_shrink) return with_blocks();
     if (worst == PSM_ERR_OOM) return fail(worst, "device arena exhausted (tables)");
     if (worst == PSM_ERR_TIMEOUT) return fail(worst, "time limit reached");
     return PSM_OK;
@@ -1196,5 +1222,5 @@ int psm_batch_polled(psm_context* ctx, const psm_graph* g, const psm_query_desc*
     return run_queries(ctx, g, qs, nq, *opt, false, results, nullptr, false, done_dev, exit_keep, poll, poll_arg);
 }
 u32 psm_context_prep_blocks_per_query(const psm_context* ctx, u32 nq) {
-    return use_cluster_batch(ctx, nq) ? (u32)ctx->batch_cluster : 1u;
+    return use_cluster_batch(ctx, nq, 0) ? (u32)ctx->batch_cluster : 1u;
 }

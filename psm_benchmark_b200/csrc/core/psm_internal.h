@@ -123,6 +123,7 @@ struct QState {
     u32 acc_words;          // words of acc / tmp
     // tables: row counts / offsets for all directed edges, concatenated
     u32* P;                 // [total_rows + 1] absolute offsets into adj
+    u32 P_rows;             // rows that P has room for (from the label frequencies)
     u32 e_row_base[PSM_MAXDIR + 1];
     u32 total_rows;
     u32* adj;               // candidate positions, allocated on the device
