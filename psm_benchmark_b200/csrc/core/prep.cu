@@ -483,6 +483,11 @@ __device__ void stage_nlf(Team& t, const DevGraph& g, QState& q, u32 need_mask, 
     }
 }
 
+// Label runs longer than this are walked by a whole warp (128 entries a round)
+// instead of the 4 or 8 lanes of a row: a hub's run of 600 entries took 20
+// dependent rounds, which set the time of a marking or table pass.
+constexpr u32 LONG_RUN = 96;
+
 // matching/FilterVertices.cpp:841-912 (generateCandidates): candidates of u
 // are the data vertices of u's label, with enough degree and NLF, adjacent to
 // a live candidate of every pivot. Marks neighbours of each pivot's
@@ -504,6 +509,22 @@ __device__ bool mark_neighbours(Team& t, const DevGraph& g, QState& q, u32 p, u3
         }
         group_label_run(g, live, c, lu, s, e);
         u32 len = e - s;
+        for (u32 m = __ballot_sync(FULL_MASK, lg == 0 && len > LONG_RUN); m; m &= m - 1) {
+            const u32 src = __ffs(m) - 1;  // a long run: the whole warp
+            const u32 s1 = __shfl_sync(FULL_MASK, s, src), e1 = __shfl_sync(FULL_MASK, e, src);
+            for (u32 j = s1 + lane; j < e1; j += 128u) {
+                u32 x[4];
+#pragma unroll
+                for (u32 k = 0; k < 4; ++k) x[k] = j + 32u * k < e1 ? __ldg(g.nbr + j + 32u * k) : 0xFFFFFFFFu;
+#pragma unroll
+                for (u32 k = 0; k < 4; ++k)
+                    if (j + 32u * k < e1) {
+                        const u32 pos = x[k] - base_u;
+                        atomicOr(out + (pos >> 5), 1u << (pos & 31u));
+                    }
+            }
+        }
+        if (len > LONG_RUN) len = 0;
         u32 mx = warp_max(len);
         for (u32 j = 0; j < mx; j += 32) {  // 4 loads in flight per lane
             u32 x[4];
@@ -833,7 +854,25 @@ __device__ bool stage_tables(Team& t, const DevGraph& g, QState& q, DevArena* ar
         }
         group_label_run<TW>(g, r < R, v, d->label[y], s, e);
         const u32 base_y = r < R ? bucket_base(g, d->label[y]) : 0;
-        u32 len = e - s, mx = warp_max(len), c = 0;
+        u32 len = e - s, c = 0;
+        for (u32 m = __ballot_sync(FULL_MASK, lg == 0 && len > LONG_RUN); m; m &= m - 1) {
+            const u32 src = __ffs(m) - 1;  // a long run: the whole warp
+            const u32 s1 = __shfl_sync(FULL_MASK, s, src), e1 = __shfl_sync(FULL_MASK, e, src);
+            const u32 b1 = __shfl_sync(FULL_MASK, base_y, src);
+            const u32* bm = q.bm[__shfl_sync(FULL_MASK, y, src)];
+            u32 hits = 0;
+            for (u32 j = s1 + lane; j < e1; j += 128u) {
+                u32 x[4];
+#pragma unroll
+                for (u32 k = 0; k < 4; ++k) x[k] = j + 32u * k < e1 ? __ldg(g.nbr + j + 32u * k) - b1 : 0u;
+#pragma unroll
+                for (u32 k = 0; k < 4; ++k) hits += j + 32u * k < e1 && test_bit(bm, x[k]);
+            }
+            hits = warp_sum(hits);
+            if (lane / TW == src / TW) c = hits;
+        }
+        if (len > LONG_RUN) len = 0;
+        const u32 mx = warp_max(len);
         for (u32 j = 0; j < mx; j += 4u * TW) {  // 4 loads in flight per lane
             u32 x[4];
 #pragma unroll
@@ -896,6 +935,35 @@ __device__ bool stage_tables(Team& t, const DevGraph& g, QState& q, DevArena* ar
             len = e - s;
         }
         u32 written = 0;
+        for (u32 m = __ballot_sync(FULL_MASK, lg == 0 && todo > LONG_RUN); m; m &= m - 1) {
+            const u32 src = __ffs(m) - 1;  // many entries, so a long run: the whole warp
+            const u32 s1 = __shfl_sync(FULL_MASK, s, src), n1 = __shfl_sync(FULL_MASK, len, src);
+            const u32 b1 = __shfl_sync(FULL_MASK, base_y, src), z1 = __shfl_sync(FULL_MASK, size_y, src);
+            const u32 y1 = __shfl_sync(FULL_MASK, y, src), t1 = __shfl_sync(FULL_MASK, todo, src);
+            u32 at = __shfl_sync(FULL_MASK, out, src);
+            const u32 stop = at + t1;
+            const u32 *bm = q.bm[y1], *rank = q.rank[y1];
+            for (u32 j = 0; at < stop; j += 128u) {
+                u32 pos[4], word[4];
+#pragma unroll
+                for (u32 k = 0; k < 4; ++k) {
+                    const u32 o = j + 32u * k + lane;
+                    pos[k] = o < n1 ? __ldg(g.nbr + s1 + o) - b1 : 0xFFFFFFFFu;
+                }
+#pragma unroll
+                for (u32 k = 0; k < 4; ++k) word[k] = pos[k] < z1 ? bm[pos[k] >> 5] : 0u;
+#pragma unroll
+                for (u32 k = 0; k < 4; ++k) {
+                    const bool hit = (word[k] >> (pos[k] & 31u)) & 1u;
+                    const u32 bal = __ballot_sync(FULL_MASK, hit);
+                    if (hit)
+                        q.adj[at + __popc(bal & ((1u << lane) - 1u))] =
+                            rank[pos[k] >> 5] + __popc(word[k] & ((1u << (pos[k] & 31u)) - 1u));
+                    at += __popc(bal);
+                }
+            }
+        }
+        if (todo > LONG_RUN) todo = 0;
         for (u32 j = 0; __any_sync(FULL_MASK, written < todo); j += 4u * TW) {  // 4 loads in flight per lane, in row order
             u32 pos[4], word[4];
 #pragma unroll
