@@ -74,9 +74,6 @@ struct psm_context {
     char* arena = nullptr;
     size_t arena_bytes = 0;
     size_t fixed_bytes = 0;       // permanent region at the start of the arena
-    DevArena* d_devarena = nullptr;
-    void* d_barrier = nullptr;
-    u32* d_ticket = nullptr;
     void* d_enum_scratch = nullptr;
     u32* d_enum_cache = nullptr;  // per-warp prefix-intersection caches (own allocation)
     int prep_threads = 512;
@@ -92,8 +89,9 @@ struct psm_context {
     u32 tune_quarters = 4;           // enumeration grid: quarters of the co-resident blocks
     u32 tune_isect = PSM_ISECT_BINARY;  // intersection variant of every enumeration launch
     cudaEvent_t ev[4]{};
-    char* pinned = nullptr;  // pinned host staging of descriptors, states and results
+    char* pinned = nullptr;  // pinned, mapped host staging of descriptors, states and results
     size_t pinned_bytes = 0;
+    std::vector<QDesc> descs;  // descriptor workspace (at most DESC_KEEP kept between runs)
     bool run_live = false;
 };
 
@@ -105,6 +103,7 @@ struct psm_run {
     QDesc* hdesc = nullptr;  // host copy (order / labels)
     u32 n = 0;
     size_t arena_free = 0;   // first arena byte not used by the run
+    std::vector<u32> P;      // host copy of the tables' row offsets (psm_run_table's first call)
 };
 
 int psm_fail(int code, const std::string& msg) { return fail(code, msg); }
@@ -135,12 +134,8 @@ int psm_run_internals(psm_run* r, RunInternals* out) {
 
 namespace {
 
-struct Layout {
-    QDesc* d_desc;
-    QState* d_q;
-    char* d_enum_q;  // per-query enumeration scratch
-    DevResult* d_res;
-};
+// Descriptors a context keeps room for between runs (36 KB each).
+constexpr size_t DESC_KEEP = 256;
 
 // Per-query device buffers and QState initialisation.
 int setup_query(psm_context* ctx, const psm_graph& g, const QDesc& d, const psm_options& opt, Bump& b,
@@ -245,7 +240,7 @@ char* staging(psm_context* ctx, size_t bytes) {
     ctx->pinned = nullptr;
     ctx->pinned_bytes = 0;
     size_t want = std::max<size_t>(bytes, 1 << 20);
-    if (cudaHostAlloc((void**)&ctx->pinned, want, cudaHostAllocDefault) != cudaSuccess) {
+    if (cudaHostAlloc((void**)&ctx->pinned, want, cudaHostAllocMapped) != cudaSuccess) {
         cudaGetLastError();
         ctx->pinned = nullptr;
         return nullptr;
@@ -264,18 +259,37 @@ int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, 
     CK(cudaSetDevice(ctx->device));
     Bump b{ctx->arena, ctx->fixed_bytes, ctx->arena_bytes};
     // descriptors
-    std::vector<QDesc> descs(nq);
+    std::vector<QDesc>& descs = ctx->descs;
+    if (descs.size() > std::max<size_t>(nq, DESC_KEEP)) {
+        descs.resize(DESC_KEEP);
+        descs.shrink_to_fit();
+    }
+    if (descs.size() < nq) descs.resize(nq);
     std::string err;
     for (u32 i = 0; i < nq; ++i) {
         int rc = psm_build_qdesc(*g, qs[i], opt, &descs[i], &err);
         if (rc) return fail(rc, "query " + std::to_string(i) + ": " + err);
     }
-    Layout lay;
-    lay.d_desc = b.take<QDesc>(nq);
-    lay.d_q = b.take<QState>(nq);
-    lay.d_enum_q = b.take<char>(psm_enum_query_bytes(nq));
-    lay.d_res = b.take<DevResult>(nq);
-    if (!lay.d_desc || !lay.d_q || !lay.d_enum_q || !lay.d_res) return fail(PSM_ERR_OOM, "device arena exhausted");
+    // Everything a run uploads lies side by side, on the host and on the device:
+    // the used prefixes of the descriptors, the states, the table allocator, the
+    // grid barrier and the batch ticket (zero). One copy per run.
+    size_t off_q = 0;
+    for (u32 i = 0; i < nq; ++i) off_q += align_up(psm_qdesc_bytes(descs[i]), 16);
+    off_q = align_up(off_q);
+    const size_t off_a = off_q + align_up(sizeof(QState) * nq), off_b = off_a + align_up(sizeof(DevArena)),
+                 up_bytes = off_b + 64 + 64, off_r = align_up(up_bytes),
+                 off_c = off_r + align_up(sizeof(DevResult) * nq);
+    char* d_up = b.take<char>(up_bytes);
+    char* d_enum_q = b.take<char>(psm_enum_query_bytes(nq));
+    if (!d_up || !d_enum_q) return fail(PSM_ERR_OOM, "device arena exhausted");
+    QState* const d_q = (QState*)(d_up + off_q);
+    DevArena* const d_devarena = (DevArena*)(d_up + off_a);
+    void* const d_barrier = d_up + off_b;
+    u32* const d_ticket = (u32*)(d_up + off_b + 64);
+    char* pin = staging(ctx, off_c + sizeof(RunBack));
+    if (!pin) return fail(PSM_ERR_OOM, "pinned host staging");
+    char* pin_dev = nullptr;  // the device's address of the staging
+    CK(cudaHostGetDevicePointer((void**)&pin_dev, pin, 0));
     // Batched preparation team: a cluster per query while the batch is small for
     // its graph (latency: a query's preparation spreads over the cluster's SMs),
     // a block per query for large batches (throughput).
@@ -294,9 +308,12 @@ int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, 
     // team scans need one word per block of the preparing team (+1)
     const u32 scan_words = grid_team ? (u32)std::max(ctx->prep_grid_blocks, ctx->cluster_size) + 1
                                      : (cluster_batch ? (u32)ctx->batch_cluster : 1u) + 1;
-    std::vector<QState> hq(nq);
-    for (u32 i = 0; i < nq; ++i) {
-        int rc = setup_query(ctx, *g, descs[i], opt, b, lay.d_desc + i, scan_words, hq[i]);
+    QState* const hq = (QState*)(pin + off_q);
+    for (size_t i = 0, o = 0; i < nq; ++i) {
+        const size_t bytes = psm_qdesc_bytes(descs[i]);
+        memcpy(pin + o, &descs[i], bytes);
+        int rc = setup_query(ctx, *g, descs[i], opt, b, (QDesc*)(d_up + o), scan_words, hq[i]);
+        o += align_up(bytes, 16);
         if (rc == PSM_ERR_OOM && may_shrink) return with_blocks();
         if (rc) return rc;
     }
@@ -308,53 +325,35 @@ int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, 
     da.base = (u32*)(ctx->arena + start);
     da.top = 0;
     da.cap = (b.cap - start) / sizeof(u32);
-    // uploads from pinned staging: descriptors (used prefix only), states,
-    // allocator; the results come back through the same buffer
-    size_t desc_bytes = 0;
-    for (u32 i = 0; i < nq; ++i) desc_bytes += align_up(psm_qdesc_bytes(descs[i]), 16);
-    const size_t off_q = align_up(desc_bytes), off_a = off_q + align_up(sizeof(QState) * nq),
-                 off_r = off_a + align_up(sizeof(DevArena)),
-                 off_c = off_r + align_up(sizeof(DevResult) * nq), off_b = off_c + align_up(psm_enum_ctl_bytes());
-    char* pin = staging(ctx, off_b + 16);
-    if (!pin) return fail(PSM_ERR_OOM, "pinned host staging");
-    {
-        size_t o = 0;
-        for (u32 i = 0; i < nq; ++i) {
-            const size_t b = psm_qdesc_bytes(descs[i]);
-            memcpy(pin + o, &descs[i], b);
-            CK(cudaMemcpyAsync(lay.d_desc + i, pin + o, b, cudaMemcpyHostToDevice, ctx->st));
-            o += align_up(b, 16);
-        }
-    }
-    memcpy(pin + off_q, hq.data(), sizeof(QState) * nq);
     memcpy(pin + off_a, &da, sizeof(da));
-    CK(cudaMemcpyAsync(lay.d_q, pin + off_q, sizeof(QState) * nq, cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(ctx->d_devarena, pin + off_a, sizeof(da), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemsetAsync(ctx->d_barrier, 0, 64, ctx->st));
-    CK(cudaMemsetAsync(ctx->d_ticket, 0, sizeof(u32), ctx->st));
+    memset(pin + off_b, 0, up_bytes - off_b);
+    CK(cudaMemcpyAsync(d_up, pin, up_bytes, cudaMemcpyHostToDevice, ctx->st));
     const u64 budget = budget_ns(opt);
     CK(cudaEventRecord(ctx->ev[0], ctx->st));
     if (grid_team && ctx->cluster_size > 0) {
-        CK(psm_launch_prep_cluster(g->dev, lay.d_q, ctx->d_devarena, ctx->cluster_size, ctx->prep_threads, ctx->st));
+        CK(psm_launch_prep_cluster(g->dev, d_q, d_devarena, ctx->cluster_size, ctx->prep_threads, ctx->st));
     } else if (grid_team) {
-        CK(psm_launch_prep_grid(g->dev, lay.d_q, ctx->d_barrier, ctx->d_devarena, budget, ctx->prep_grid_blocks,
+        CK(psm_launch_prep_grid(g->dev, d_q, d_barrier, d_devarena, budget, ctx->prep_grid_blocks,
                                 ctx->prep_threads, ctx->st));
     } else if (cluster_batch) {
         const int clusters = std::min<int>(ctx->batch_clusters, (int)nq);
-        CK(psm_launch_prep_cluster_batch(g->dev, lay.d_q, nq, ctx->d_ticket, ctx->d_devarena, ctx->batch_cluster,
+        CK(psm_launch_prep_cluster_batch(g->dev, d_q, nq, d_ticket, d_devarena, ctx->batch_cluster,
                                          clusters, ctx->prep_threads, ctx->st));
     } else {
         int blocks = std::min<int>(ctx->prep_block_blocks, (int)nq);
-        CK(psm_launch_prep_block(g->dev, lay.d_q, nq, ctx->d_ticket, ctx->d_devarena, blocks, ctx->prep_threads,
+        CK(psm_launch_prep_block(g->dev, d_q, nq, d_ticket, d_devarena, blocks, ctx->prep_threads,
                                  ctx->st));
     }
     CK(cudaEventRecord(ctx->ev[1], ctx->st));
     if (!prep_only)
-        CK(psm_launch_enum(g->dev, lay.d_q, nq, ctx->d_enum_scratch, lay.d_enum_q, budget, opt.emit ? 1 : 0,
+        CK(psm_launch_enum(g->dev, d_q, nq, ctx->d_enum_scratch, d_enum_q, budget, opt.emit ? 1 : 0,
                            grid_team ? ctx->enum_blocks : batch_enum_blocks(ctx), ctx->d_enum_cache, done, exit_keep,
                            ctx->st, grid_team ? 8u : ctx->tune_grabs, ctx->tune_isect));
     CK(cudaEventRecord(ctx->ev[2], ctx->st));
-    CK(psm_launch_gather(lay.d_q, nq, lay.d_res, ctx->st));
+    // results, the enumeration's counters and GridBarrier::abort (the barrier's
+    // second word) go straight to the staging: one synchronisation, no copies
+    CK(psm_launch_gather(d_q, nq, (DevResult*)(pin_dev + off_r), ctx->st, prep_only ? nullptr : ctx->d_enum_scratch,
+                         grid_team ? (u32*)d_barrier + 1 : nullptr, (RunBack*)(pin_dev + off_c)));
     if (poll) {
         // the caller collects per-query completion records while the launch runs
         cudaError_t q;
@@ -365,23 +364,15 @@ int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, 
         if (q != cudaSuccess) return cuda_fail(q, "batch launch");
         poll(poll_arg);
     }
-    std::vector<DevResult> res(nq);
-    CK(cudaMemcpyAsync(pin + off_r, lay.d_res, sizeof(DevResult) * nq, cudaMemcpyDeviceToHost, ctx->st));
-    // the enumerator's control block and the grid barrier's abort word come
-    // back through the staging buffer too: one synchronisation per run
-    if (!prep_only) CK(psm_enum_copy_ctl(ctx->d_enum_scratch, pin + off_c, ctx->st));
-    if (grid_team)  // GridBarrier::abort (second word of the barrier)
-        CK(cudaMemcpyAsync(pin + off_b, (char*)ctx->d_barrier + 4, sizeof(u32), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    EnumStats es{};
-    if (!prep_only) psm_enum_ctl_stats(pin + off_c, &es);
-    memcpy(res.data(), pin + off_r, sizeof(DevResult) * nq);
+    const RunBack back = *(const RunBack*)(pin + off_c);
+    const EnumStats es = back.es;
+    const DevResult* const res = (const DevResult*)(pin + off_r);
     const u32 enum_err = es.error;
     float prep_ms = 0, enum_ms = 0;
     CK(cudaEventElapsedTime(&prep_ms, ctx->ev[0], ctx->ev[1]));
     CK(cudaEventElapsedTime(&enum_ms, ctx->ev[1], ctx->ev[2]));
-    u64 h2d = sizeof(QState) * (u64)nq + sizeof(DevArena) + 64 + 4, d2h = sizeof(DevResult) * (u64)nq + (prep_only ? 0 : psm_enum_ctl_bytes()) + (grid_team ? 4 : 0);
-    for (u32 i = 0; i < nq; ++i) h2d += psm_qdesc_bytes(descs[i]);
+    const u64 h2d = up_bytes, d2h = sizeof(DevResult) * (u64)nq + sizeof(RunBack);
     int worst = PSM_OK;
     for (u32 i = 0; i < nq; ++i) {
         fill_result(res[i], prep_ms, enum_ms, es.donations, &results[i]);
@@ -393,9 +384,7 @@ int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, 
         if (results[i].status != PSM_OK && worst == PSM_OK) worst = (int)results[i].status;
     }
     if (grid_team) {
-        u32 ab = 0;
-        memcpy(&ab, pin + off_b, sizeof(u32));
-        if (ab) {
+        if (back.abort) {
             for (u32 i = 0; i < nq; ++i) results[i].status = PSM_ERR_INTERNAL;
             worst = PSM_ERR_INTERNAL;
         }
@@ -403,7 +392,7 @@ int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, 
     if (hq[0].trace && nq > 1) {
         // per-query time at which the cap was reached, relative to the first
         std::vector<QState> st(nq);
-        CK(cudaMemcpy(st.data(), lay.d_q, sizeof(QState) * nq, cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(st.data(), d_q, sizeof(QState) * nq, cudaMemcpyDeviceToHost));
         u64 t0 = ~0ull;
         for (auto& s : st)
             if (s.done_ns) t0 = std::min(t0, s.done_ns);
@@ -428,13 +417,13 @@ int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, 
     if (keep) {
         keep->ctx = ctx;
         keep->g = g;
-        keep->d_q = lay.d_q;
-        CK(cudaMemcpy(&keep->hq, lay.d_q, sizeof(QState), cudaMemcpyDeviceToHost));
+        keep->d_q = d_q;
+        CK(cudaMemcpy(&keep->hq, d_q, sizeof(QState), cudaMemcpyDeviceToHost));
         keep->hdesc = new QDesc;
         memcpy(keep->hdesc, &descs[0], sizeof(QDesc));
         keep->n = descs[0].n;
         DevArena top{};
-        CK(cudaMemcpy(&top, ctx->d_devarena, sizeof(top), cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(&top, d_devarena, sizeof(top), cudaMemcpyDeviceToHost));
         keep->arena_free = align_up(start + (size_t)std::min<u64>(top.top, top.cap) * sizeof(u32));
         ctx->run_live = true;
     }
@@ -548,9 +537,6 @@ int psm_context_create(int device, uint64_t arena_bytes, psm_context** out) {
         return cuda_fail(e, "context allocation");
     }
     Bump b{c->arena, 0, arena_bytes};
-    c->d_devarena = b.take<DevArena>(1);
-    c->d_barrier = b.take<char>(64);
-    c->d_ticket = b.take<u32>(1);
     c->d_enum_scratch = b.take<char>(psm_enum_scratch_bytes());
     c->fixed_bytes = b.top;
     if (psm_prep_grid_max_blocks(c->prep_threads, &c->prep_grid_blocks) != cudaSuccess ||
@@ -762,9 +748,13 @@ int psm_run_table(psm_run* r, uint32_t a, uint32_t b, uint32_t* offsets, uint32_
     if (!((d.adj[a] >> b) & 1u)) return fail(PSM_ERR_ARG, "not a query edge");
     if (r->hq.adj == nullptr) return fail(PSM_ERR_ARG, "tables were not built (empty candidate set)");
     u32 e = d.e_first[a] + (u32)__builtin_popcount(d.adj[a] & ((1u << b) - 1u));
-    u32 base = r->hq.e_row_base[e], R = r->hq.cnt[a];
-    std::vector<u32> P(R + 1);
-    CK(cudaMemcpy(P.data(), r->hq.P + base, (R + 1) * sizeof(u32), cudaMemcpyDeviceToHost));
+    const u32 base = r->hq.e_row_base[e], R = r->hq.cnt[a];
+    if (r->P.empty()) {  // the row offsets of all tables at once: they do not change
+        std::vector<u32> all((size_t)r->hq.total_rows + 1);
+        CK(cudaMemcpy(all.data(), r->hq.P, all.size() * sizeof(u32), cudaMemcpyDeviceToHost));
+        r->P = std::move(all);
+    }
+    const u32* P = r->P.data() + base;
     u32 z = P[R] - P[0];
     if (rows) *rows = R;
     if (nnz) *nnz = z;

@@ -1204,13 +1204,6 @@ __device__ bool periodic(QState& q, u32 qi, WarpStack* ws, u32 d, u32 d0, u32& i
     return __shfl_sync(FULL_MASK, stop, 0) != 0;
 }
 
-// count += c * w; false when that passes 2^64 - 1.
-__device__ __forceinline__ bool add_weighted(u64& count, u64 c, u64 w) {
-    const u64 x = c * w;
-    count += x;
-    return __umul64hi(c, w) == 0 && count >= x;
-}
-
 // Depth-first search below the prefix ws->pos[0, d0). With `enter` the walked
 // vertex of depth d0 - 1 was just placed (its weight and the level d0 are set up
 // here), otherwise the level d0 has been set up (driver range in ws). Returns
@@ -1751,7 +1744,16 @@ __global__ void enum_init_kernel(QState* qs, u32 nq, EnumCtl* ctl, Slot* slots, 
     for (u32 i = threadIdx.x; i < QCAP; i += blockDim.x) slots[i].seq = i;
 }
 
-__global__ void gather_kernel(QState* qs, u32 nq, DevResult* out) {
+// Per-query results and the launch's counters; `out` and `back` may be mapped
+// host memory (one kernel instead of a kernel and three copies per run).
+__global__ void gather_kernel(QState* qs, u32 nq, DevResult* out, const EnumCtl* ctl, const u32* abort_word,
+                              RunBack* back) {
+    if (back && blockIdx.x == 0 && threadIdx.x == 0) {
+        RunBack b{};
+        if (ctl) b.es = EnumStats{ctl->error, ctl->donations, ctl->tasks, ctl->idle_polls};
+        if (abort_word) b.abort = *abort_word;
+        *back = b;
+    }
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += gridDim.x * blockDim.x) {
         QState& q = qs[i];
         DevResult r;
@@ -1774,9 +1776,10 @@ size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 }  // namespace
 
-cudaError_t psm_launch_gather(QState* qs, u32 nq, DevResult* out, cudaStream_t st) {
+cudaError_t psm_launch_gather(QState* qs, u32 nq, DevResult* out, cudaStream_t st, const void* enum_scratch,
+                              const u32* abort_word, RunBack* back) {
     u32 blocks = (nq + 255) / 256;
-    gather_kernel<<<blocks ? blocks : 1, 256, 0, st>>>(qs, nq, out);
+    gather_kernel<<<blocks ? blocks : 1, 256, 0, st>>>(qs, nq, out, (const EnumCtl*)enum_scratch, abort_word, back);
     return cudaGetLastError();
 }
 
@@ -1830,24 +1833,6 @@ cudaError_t psm_enum_max_blocks(int* blocks) {
     if (e != cudaSuccess) return e;
     *blocks = sms * (per_sm < 1 ? 1 : per_sm);
     return cudaSuccess;
-}
-
-// Size of the launch-wide control block (error flag, scheduling counters).
-size_t psm_enum_ctl_bytes() { return sizeof(EnumCtl); }
-
-// Queues a copy of the control block into host memory (pinned staging).
-cudaError_t psm_enum_copy_ctl(const void* scratch, void* host, cudaStream_t st) {
-    return cudaMemcpyAsync(host, scratch, sizeof(EnumCtl), cudaMemcpyDeviceToHost, st);
-}
-
-// Decodes a control block copied by psm_enum_copy_ctl.
-void psm_enum_ctl_stats(const void* host, EnumStats* out) {
-    EnumCtl h;
-    memcpy(&h, host, sizeof(h));
-    out->error = h.error;
-    out->donations = h.donations;
-    out->tasks = h.tasks;
-    out->idle_polls = h.idle_polls;
 }
 
 // Reads back the launch-wide error flag and scheduling counters.

@@ -107,12 +107,10 @@ cudaError_t psm_launch_enum(const DevGraph& g, QState* qs, u32 nq, void* scratch
                             int emit, int blocks, u32* cache, QDoneRec* done, u32 exit_keep, cudaStream_t st,
                             u32 grabs_per_warp = 8, u32 isect = 0);
 cudaError_t psm_enum_max_blocks(int* blocks);
-cudaError_t psm_launch_gather(QState* qs, u32 nq, DevResult* out, cudaStream_t st);
+// back (optional): also the counters of enum_scratch and *abort_word (each may be
+// null). out and back may be mapped host memory.
+cudaError_t psm_launch_gather(QState* qs, u32 nq, DevResult* out, cudaStream_t st, const void* enum_scratch = nullptr,
+                              const u32* abort_word = nullptr, RunBack* back = nullptr);
 cudaError_t psm_enum_read_ctl(void* scratch, EnumStats* out, cudaStream_t st);
-// Split form for callers with pinned staging: queue the control block's copy
-// on the stream, then read the stats once the stream has synchronised.
-size_t psm_enum_ctl_bytes();
-cudaError_t psm_enum_copy_ctl(const void* scratch, void* host, cudaStream_t st);
-void psm_enum_ctl_stats(const void* host, EnumStats* out);
 cudaError_t psm_launch_unit_plan(const DevGraph& g, QState* qs, u32 nq, cudaStream_t st);
 cudaError_t psm_launch_unit_emit(QState* qs, u32 nq, u32* const* bufs, const u64* caps, cudaStream_t st);

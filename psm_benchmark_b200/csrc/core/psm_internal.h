@@ -240,6 +240,13 @@ struct EnumStats {
     u64 donations, tasks, idle_polls;
 };
 
+// What a run brings back beside its results: the enumeration's counters and the
+// grid barrier's abort word.
+struct RunBack {
+    EnumStats es;
+    u32 abort;
+};
+
 // Device-side bump allocator over an arena region.
 struct DevArena {
     u64 base_words;          // unused, keeps the struct 16-byte sized
