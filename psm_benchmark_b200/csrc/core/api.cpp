@@ -866,23 +866,27 @@ int join_rels(psm_context* ctx, Arena2& ar, const u32* label, const Rel& B, cons
     JoinTable t{};
     t.mask = (u32)(cap - 1);
     t.slots = ar.high<u32>(cap);
-    t.gcount = ar.high<u32>(cap);
-    t.gfill = ar.high<u32>(cap);
+    // zeroed with one memset: the counters of every slot, then the join's words
+    char* zero = ar.high<char>(2 * sizeof(u32) * cap + sizeof(JoinWords));
+    t.gcount = (u32*)zero;
+    t.gfill = t.gcount + cap;
+    t.words = (JoinWords*)(zero + 2 * sizeof(u32) * cap);
     t.goff = ar.high<u64>(cap);
     t.grp = ar.high<u32>(B.n);
     t.members = ar.high<u32>(B.n);
-    t.scan_tmp = ar.high<u64>(psm_scan_tmp_bytes(cap) / sizeof(u64) + 1);
-    t.error = ar.high<u32>(1);
-    u64* d_total = ar.high<u64>(1);
-    if (!t.slots || !t.gcount || !t.gfill || !t.goff || !t.grp || !t.members || !t.scan_tmp || !t.error || !d_total)
+    if (!t.slots || !zero || !t.goff || !t.grp || !t.members)
         return fail(PSM_ERR_OOM, "device arena exhausted (join table)");
     CK(psm_join_build(B.rows, B.n, sp, t, ctx->st));
-    CK(cudaMemsetAsync(d_total, 0, sizeof(u64), ctx->st));
+    u64* const d_total = &t.words->total;
+    JoinWords words{};
     u64 n_out = 0;
     if (count_only) {
         CK(psm_join_probe(P.rows, P.n, B.rows, sp, t, nullptr, nullptr, nullptr, (unsigned long long*)d_total,
                           ctx->st));
-        CK(cudaMemcpyAsync(&n_out, d_total, sizeof(u64), cudaMemcpyDeviceToHost, ctx->st));
+        CK(cudaMemcpyAsync(&words, t.words, sizeof(words), cudaMemcpyDeviceToHost, ctx->st));
+        CK(cudaStreamSynchronize(ctx->st));
+        if (words.error) return fail(PSM_ERR_INTERNAL, "join table overflow");
+        n_out = words.total;
     } else {
         u32* cnt = ar.high<u32>(P.n);
         u64* off = ar.high<u64>(P.n);
@@ -890,8 +894,10 @@ int join_rels(psm_context* ctx, Arena2& ar, const u32* label, const Rel& B, cons
         if (!cnt || !off || !stmp) return fail(PSM_ERR_OOM, "device arena exhausted (join counts)");
         CK(psm_join_probe(P.rows, P.n, B.rows, sp, t, cnt, nullptr, nullptr, nullptr, ctx->st));
         CK(psm_excl_scan(cnt, P.n, off, stmp, d_total, ctx->st));
-        CK(cudaMemcpyAsync(&n_out, d_total, sizeof(u64), cudaMemcpyDeviceToHost, ctx->st));
-        CK(cudaStreamSynchronize(ctx->st));
+        CK(cudaMemcpyAsync(&words, t.words, sizeof(words), cudaMemcpyDeviceToHost, ctx->st));
+        CK(cudaStreamSynchronize(ctx->st));  // the only wait: the size of the output
+        if (words.error) return fail(PSM_ERR_INTERNAL, "join table overflow");
+        n_out = words.total;
         out->ncols = P.ncols + sp.nbx;
         for (u32 j = 0; j < P.ncols; ++j) out->vert[j] = P.vert[j];
         for (u32 x = 0; x < sp.nbx; ++x) out->vert[P.ncols + x] = B.vert[sp.bx[x]];
@@ -900,10 +906,6 @@ int join_rels(psm_context* ctx, Arena2& ar, const u32* label, const Rel& B, cons
         if (!out->rows) return fail(PSM_ERR_OOM, "device arena exhausted (joined rows)");
         CK(psm_join_probe(P.rows, P.n, B.rows, sp, t, nullptr, out->rows, off, nullptr, ctx->st));
     }
-    u32 err = 0;
-    CK(cudaMemcpyAsync(&err, t.error, sizeof(u32), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    if (err) return fail(PSM_ERR_INTERNAL, "join table overflow");
     *total = n_out;
     *peak_bytes = std::max<u64>(*peak_bytes, ar.lo + (hi0 - ar.hi));
     ar.hi = hi0;
@@ -1199,6 +1201,7 @@ int psm_hash_join(psm_context* ctx, const uint32_t* r_rows, uint64_t r_n, uint32
     if (out_cols) *out_cols = out.ncols;
     if (out_vertex)
         for (u32 i = 0; i < out.ncols; ++i) out_vertex[i] = out.vert[i];
+    CK(cudaStreamSynchronize(ctx->st));  // the rows are still being written
     if (out_capacity < total) return fail(PSM_ERR_ARG, "output buffer too small");
     if (total) CK(cudaMemcpy(out_rows, out.rows, total * out.ncols * sizeof(u32), cudaMemcpyDeviceToHost));
     return PSM_OK;

@@ -77,6 +77,20 @@ __global__ void hj_build(const u32* __restrict__ brows, u64 nb, JoinSpec sp, u32
     }
 }
 
+// Gives every key with rows its place among the members, in any order: one
+// cursor update per warp instead of a scan over the slots (three launches).
+__global__ void hj_offsets(u64 slots, const u32* gcount, u64* goff, u64* cursor) {
+    const u32 lane = lane_id();
+    for (u64 b = blockIdx.x * (u64)blockDim.x + (threadIdx.x & ~31u); b < slots; b += (u64)gridDim.x * blockDim.x) {
+        const u64 i = b + lane;
+        const u32 c = i < slots ? gcount[i] : 0u, incl = warp_incl_scan(c);
+        u64 at = 0;
+        if (lane == 31 && incl) at = atomicAdd((unsigned long long*)cursor, (unsigned long long)incl);
+        at = __shfl_sync(FULL_MASK, at, 31);
+        if (c) goff[i] = at + incl - c;
+    }
+}
+
 __global__ void hj_scatter(u64 nb, const u32* grp, const u64* goff, u32* gfill, u32* members) {
     for (u64 i = blockIdx.x * (u64)blockDim.x + threadIdx.x; i < nb; i += (u64)gridDim.x * blockDim.x) {
         const u32 h = grp[i];
@@ -151,6 +165,42 @@ __global__ void scan_tiles(const u32* in, u64 n, u64* tile_sum) {
         v = warp_sum64(v);
         if (threadIdx.x == 0) tile_sum[blockIdx.x] = v;
     }
+}
+
+// Exclusive scan of a few tiles by one block, in one launch.
+__global__ void scan_few(const u32* in, u64 n, u64* out, u64* total) {
+    __shared__ u64 wsum[32];
+    __shared__ u64 carry;
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    const u32 lane = lane_id(), w = threadIdx.x >> 5;
+    for (u64 b = 0; b < n; b += blockDim.x) {
+        const u64 i = b + threadIdx.x;
+        const u64 x = i < n ? in[i] : 0;
+        u64 incl = x;
+        for (int o = 1; o < 32; o <<= 1) {
+            const u64 y = __shfl_up_sync(FULL_MASK, incl, o);
+            if (lane >= (u32)o) incl += y;
+        }
+        if (lane == 31) wsum[w] = incl;
+        __syncthreads();
+        if (w == 0) {
+            const u64 v = lane < (blockDim.x >> 5) ? wsum[lane] : 0;
+            u64 vi = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const u64 y = __shfl_up_sync(FULL_MASK, vi, o);
+                if (lane >= (u32)o) vi += y;
+            }
+            wsum[lane] = vi - v;
+        }
+        __syncthreads();
+        const u64 excl = carry + wsum[w] + incl - x;
+        __syncthreads();
+        if (i < n) out[i] = excl;
+        if (threadIdx.x == blockDim.x - 1) carry = excl + x;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0 && total) *total = carry;
 }
 
 // One block: exclusive scan of the tile sums in place; total at [ntiles].
@@ -236,8 +286,13 @@ int grid_for(u64 n, int threads) {
 size_t psm_scan_tmp_bytes(u64 n) { return sizeof(u64) * ((n + SCAN_TILE - 1) / SCAN_TILE + 2); }
 
 cudaError_t psm_excl_scan(const u32* in, u64 n, u64* out, u64* tmp, u64* total_dev, cudaStream_t st) {
+    // Up to SCAN_FEW tiles one block scans in about the time of one launch (4,096
+    // items a round of ~2 us); beyond, three launches over all tiles.
+    constexpr u64 SCAN_FEW = 2;
     const u64 ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    if (ntiles > 0) {
+    if (ntiles > 0 && ntiles <= SCAN_FEW) {
+        scan_few<<<1, SCAN_THREADS, 0, st>>>(in, n, out, total_dev);
+    } else if (ntiles > 0) {
         scan_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, st>>>(in, n, tmp);
         scan_tile_sums<<<1, SCAN_THREADS, 0, st>>>(tmp, ntiles);
         scan_apply<<<(unsigned)ntiles, SCAN_THREADS, 0, st>>>(in, n, tmp, out);
@@ -250,14 +305,13 @@ cudaError_t psm_excl_scan(const u32* in, u64 n, u64* out, u64* tmp, u64* total_d
 
 cudaError_t psm_join_build(const u32* brows, u64 nb, const JoinSpec& sp, const JoinTable& t, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(t.slots, 0xFF, sizeof(u32) * (t.mask + 1ull), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(t.gcount, 0, sizeof(u32) * (t.mask + 1ull), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(t.gfill, 0, sizeof(u32) * (t.mask + 1ull), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(t.error, 0, sizeof(u32), st);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(t.gcount, 0, 2 * sizeof(u32) * (t.mask + 1ull) + sizeof(JoinWords), st);
     if (e != cudaSuccess) return e;
-    if (nb) hj_build<<<grid_for(nb, 256), 256, 0, st>>>(brows, nb, sp, t.slots, t.mask, t.grp, t.gcount, t.error);
-    e = psm_excl_scan(t.gcount, t.mask + 1ull, t.goff, t.scan_tmp, nullptr, st);
-    if (e != cudaSuccess) return e;
-    if (nb) hj_scatter<<<grid_for(nb, 256), 256, 0, st>>>(nb, t.grp, t.goff, t.gfill, t.members);
+    if (nb == 0) return cudaSuccess;
+    hj_build<<<grid_for(nb, 256), 256, 0, st>>>(brows, nb, sp, t.slots, t.mask, t.grp, t.gcount, &t.words->error);
+    hj_offsets<<<grid_for(t.mask + 1ull, 256), 256, 0, st>>>(t.mask + 1ull, t.gcount, t.goff, &t.words->cursor);
+    hj_scatter<<<grid_for(nb, 256), 256, 0, st>>>(nb, t.grp, t.goff, t.gfill, t.members);
     return cudaGetLastError();
 }
 

@@ -17,17 +17,25 @@ struct JoinSpec {
     u32 bx_same[PSM_MAXQ];         // per bx column: probe columns with the same label (bit mask)
 };
 
+// Counters of one join, read back with one copy.
+struct JoinWords {
+    u64 total;      // output rows
+    u64 cursor;     // members handed out to groups
+    u32 error;      // set if a key could not be placed
+    u32 pad;
+};
+
 // Device buffers of one build side: 2^k slots (mask = 2^k - 1) and nb rows.
 struct JoinTable {
     u32 mask;
     u32* slots;     // [mask+1] first build row of a key, or 0xFFFFFFFF
+    // one zeroed block: gcount, gfill, words
     u32* gcount;    // [mask+1] rows per key
     u32* gfill;     // [mask+1] scatter cursors
-    u64* goff;      // [mask+1] exclusive scan of gcount
+    JoinWords* words;
+    u64* goff;      // [mask+1] first member of each key with rows
     u32* grp;       // [nb] slot of each build row
     u32* members;   // [nb] build rows grouped by key
-    u64* scan_tmp;  // psm_scan_tmp_bytes(mask+1)
-    u32* error;     // set if a key could not be placed
 };
 
 size_t psm_scan_tmp_bytes(u64 n);
