@@ -403,14 +403,16 @@ def ours_arm(args, world, rank, local):
                          # algorithmic bytes per launch of this run
                          "traffic": enum_traffic(), "alg_bytes_per_launch": alg / (nq * args.steps),
                          "numerator": "reference-equivalent intersection bytes, scaled to the cap on queries "
-                                      "counted past it (bytes x cap / unclamped count)",
+                                      "counted past it (bytes x cap / unclamped count); counted vertices "
+                                      "multiply instead of being read, so the kernel moves a fraction of this "
+                                      "volume and frac may pass 1",
                          "counted_past_cap": internal / max(1, sum(counts) * args.steps) - 1.0,
                          # what the captures show bounds the kernel: its rows
                          # stay in L1/L2, so DRAM carries a sliver of the
                          # algorithmic bytes and instruction issue sets the time
-                         "limiter": "instruction issue and latency on L1/L2-resident rows (ncu: DRAM bytes "
-                                    "about 1/2000 of the algorithmic bytes, L1 hit 97.5 %, 20.5 of 32 threads "
-                                    "active per instruction; profiles/enum_kernel_q32_plain_rmat_s20.md)"},
+                         "limiter": "instruction issue and latency on L1/L2-resident rows (ncu: 50 % of the issue "
+                                    "slots, L1 hit 95.7 %, 21.8 of 32 threads active, DRAM 0.02 %; "
+                                    "profiles/enum_kernel_long_search_rmat_s20.md)"},
             "clocks": clk}
     # Batched path on the same queries: one preparation launch + one
     # enumeration launch for the whole step (device time, CUDA events).

@@ -1220,16 +1220,17 @@ __device__ void cfl_order_select(QState& q, const u32* pw) {
 //  - it does not share the label of the last walked vertex when it precedes
 //    that one in the order (the lanes try that vertex's candidates side by
 //    side, so a hit would differ from lane to lane);
-//  - the product of the counted vertices' candidate counts stays below 2^52,
-//    so that no weight overflows: the vertices of the largest estimated
-//    fan-out |C(u)| x prod_b nnz(b, u) / (|C(b)||C(u)|) are taken first.
+//  - the product of the counted vertices' candidate counts stays below 2^48,
+//    so that no product of a step overflows (a memoised level adds 15 bits):
+//    the vertices of the largest estimated fan-out
+//    |C(u)| x prod_b nnz(b, u) / (|C(b)||C(u)|) are taken first.
 // Measured (B200, enumeration only, walking every vertex -> this rule): 160
 // queries of 4-32 vertices on the scale-20 graph in one batch 480 -> 70 ms; 16
 // 12-vertex queries one by one 25.1 -> 4.9 ms, nine of 24-32 vertices 31.6 ->
 // 3.1 ms. One warp, lane = place in the matching order; returns, for a counted
 // place of ord, the number of walked depths before it (~0 for a walked one).
 __device__ u32 sink_plan_warp(QState& q, bool may_count) {
-    constexpr float MAX_BITS = 52.f;
+    constexpr float MAX_BITS = 48.f;
     const QDesc* d = q.desc;
     const u32 n = q.n_enum;
     const u32 lane = lane_id();
