@@ -139,7 +139,7 @@ constexpr size_t DESC_KEEP = 256;
 
 // Per-query device buffers and QState initialisation.
 int setup_query(psm_context* ctx, const psm_graph& g, const QDesc& d, const psm_options& opt, Bump& b,
-                QDesc* d_desc, u32 scan_words, QState& q) {
+                QDesc* d_desc, u32 scan_words, u32 naccs, QState& q) {
     memset(&q, 0, sizeof(q));
     q.desc = d_desc;
     u32 maxw = 1, maxb = 1;
@@ -157,9 +157,10 @@ int setup_query(psm_context* ctx, const psm_graph& g, const QDesc& d, const psm_
     u64 rows = 0;
     for (u32 x = 0; x < d.n; ++x) rows += (u64)g.freq(d.label[x]) * (d.e_first[x + 1] - d.e_first[x]);
     if (rows >= 0xFFFFFFF0ull) return fail(PSM_ERR_ARG, "candidate tables too large for 32-bit offsets");
-    q.acc = b.take<u32>(maxw);
-    q.tmp = b.take<u32>(maxw);
+    q.acc = b.take<u32>((size_t)naccs * maxw);
+    q.tmp = q.acc + maxw;
     q.acc_words = maxw;
+    q.naccs = naccs;
     q.P = b.take<u32>(rows + 1);
     q.P_rows = (u32)rows;
     q.scan = b.take<u32>((size_t)scan_words * std::max(d.n, 1u));  // multi_compact: a block's word per vertex
@@ -171,7 +172,7 @@ int setup_query(psm_context* ctx, const psm_graph& g, const QDesc& d, const psm_
         q.est_out = b.take<u64>(PSM_PLAN_WORDS);
         if (!q.est_a || !q.est_out) return fail(PSM_ERR_OOM, "device arena exhausted (estimates)");
     }
-    if (!q.acc || !q.tmp || !q.P || !q.scan) return fail(PSM_ERR_OOM, "device arena exhausted (tables)");
+    if (!q.acc || !q.P || !q.scan) return fail(PSM_ERR_OOM, "device arena exhausted (tables)");
     q.cap = opt.cap;
     // Diagnostics: PSM_TRACE=1 records a device timestamp per preparation
     // step (printed to stderr); PSM_HYBRID=1 lets block 0 of the plain-path
@@ -312,7 +313,7 @@ int run_queries(psm_context* ctx, const psm_graph* g, const psm_query_desc* qs, 
     for (size_t i = 0, o = 0; i < nq; ++i) {
         const size_t bytes = psm_qdesc_bytes(descs[i]);
         memcpy(pin + o, &descs[i], bytes);
-        int rc = setup_query(ctx, *g, descs[i], opt, b, (QDesc*)(d_up + o), scan_words, hq[i]);
+        int rc = setup_query(ctx, *g, descs[i], opt, b, (QDesc*)(d_up + o), scan_words, grid_team ? PSM_ACCS : 2u, hq[i]);
         o += align_up(bytes, 16);
         if (rc == PSM_ERR_OOM && may_shrink) return with_blocks();
         if (rc) return rc;

@@ -137,6 +137,21 @@ void fill_filter_plan(const QGraph& q, u32 root, FilterPlan& fp) {
     for (int i = (int)levels - 2; i >= 0; --i)
         for (u32 j = lo[i]; j < lo[i + 1]; ++j)
             if (under[t.order[j]]) add(STEP_PRUNE, t.order[j], under[t.order[j]]);
+    // groups of consecutive independent steps (a step reads its pivots, writes its vertex)
+    for (u32 s = 0; s < fp.nsteps;) {
+        const u32 kind = fp.step_kind[s];
+        u32 writes = 1u << fp.step_u[s], reads = fp.step_mask[s], pivots = (u32)__builtin_popcount(reads), c = 1;
+        for (; s + c < fp.nsteps && fp.step_kind[s + c] == kind; ++c) {
+            const u32 w = 1u << fp.step_u[s + c], r = fp.step_mask[s + c];
+            pivots += (u32)__builtin_popcount(r);
+            if ((r & writes) || (w & (reads | writes)) || (kind == STEP_GEN && pivots > PSM_ACCS)) break;
+            writes |= w;
+            reads |= r;
+            fp.step_group[s + c] = 0;
+        }
+        fp.step_group[s] = c;
+        s += c;
+    }
 }
 
 void core_paths(const QGraph& q, const Tree& t, u32 u, std::vector<u32>& cur, std::vector<std::vector<u32>>& out) {
@@ -310,6 +325,15 @@ int psm_build_qdesc(const psm_graph& g, const psm_query_desc& qd, const psm_opti
         d->adj[u] = adj[u];
         d->item_label[u] = q.lab[u];
         d->item_deg[u] = q.deg(u);
+    }
+    u32 group = 0;
+    for (u32 s = 0; s < 2 * n; ++s) {
+        const u32 u = s % n;
+        if (s && !(group & (adj[u] | 1u << u)))
+            d->refine_join |= 1ull << s;
+        else
+            group = 0;
+        group |= 1u << u;
     }
     std::vector<u32> lab, cnt, grp;
     d->nlf_off[0] = 0;

@@ -483,6 +483,15 @@ __device__ void stage_nlf(Team& t, const DevGraph& g, QState& q, u32 need_mask, 
     }
 }
 
+// This warp's number when the team's numbering starts at warp `first`: the
+// passes that share a barrier interval start at different warps, so that short
+// ones run side by side.
+template <class Team>
+__device__ __forceinline__ u32 warp_from(const Team& t, u32 first) {
+    const u32 n = t.nwarps(), w = t.warp() + n - first % n;
+    return w >= n ? w - n : w;
+}
+
 // Label runs longer than this are walked by a whole warp (128 entries a round)
 // instead of the 4 or 8 lanes of a row: a hub's run of 600 entries took 20
 // dependent rounds, which set the time of a marking or table pass.
@@ -494,12 +503,12 @@ constexpr u32 LONG_RUN = 96;
 // candidates into a bucket bitmap (8 lanes per candidate), ANDs across
 // pivots, then applies the degree + NLF test per surviving bit.
 template <class Team>
-__device__ bool mark_neighbours(Team& t, const DevGraph& g, QState& q, u32 p, u32 lu, u32* out) {
+__device__ bool mark_neighbours(Team& t, const DevGraph& g, QState& q, u32 p, u32 lu, u32* out, u32 first_warp = 0) {
     const u32 lane = lane_id(), grp = lane >> 3, lg = lane & 7u;
     const u32 base_u = bucket_base(g, lu);
     const u32 base_p = bucket_base(g, q.desc->label[p]);
     const u32 N = q.cnt[p];
-    for (u32 i0 = t.warp() * 4u; i0 < N; i0 += t.nwarps() * 4u) {
+    for (u32 i0 = warp_from(t, first_warp) * 4u; i0 < N; i0 += t.nwarps() * 4u) {
         u32 i = i0 + grp;
         u32 c = 0, s, e;
         bool live = false;
@@ -618,6 +627,47 @@ __device__ __forceinline__ void append_word(const DevGraph& g, QState& q, u32 u,
     for (; x; x &= x - 1) q.list[u][at++] = base + __ffs(x) - 1u;
 }
 
+// A group of generate steps by the whole grid (FilterPlan::step_group; every
+// vertex's NLF set is in its bitmap already, QState::nlf_all). All pivots of all
+// steps are marked in one barrier interval, each into a bitmap of its own, and
+// all steps' sets are formed in the next. The lists keep the order in which
+// warps append to them until the filter's end sorts them (no step before
+// depends on it). A step of its own took two to four intervals and the ordered
+// compaction's two: the filter steps of a 12-vertex query on the scale-20 graph
+// 300 us, now 135 us; preparing a 31-vertex query 1.05 -> 0.76 ms.
+template <class Team>
+__device__ bool generate_group(Team& t, const DevGraph& g, QState& q, const FilterPlan& fp, u32 s0, u32 count) {
+    u32 marks = 0, total = 0;
+    for (u32 s = s0; s < s0 + count; ++s) total += __popc(fp.step_mask[s]);
+    for (u32 s = s0; s < s0 + count; ++s)
+        for (u32 pm = fp.step_mask[s]; pm; pm &= pm - 1, ++marks)
+            mark_neighbours(t, g, q, (u32)__ffs(pm) - 1, q.desc->label[fp.step_u[s]], q.acc + marks * q.acc_words,
+                            marks * (t.nwarps() / total));
+    TSYNC_B(t);
+    marks = 0;
+    u32 first_warp = 0;
+    for (u32 s = s0; s < s0 + count; ++s) {
+        const u32 u = fp.step_u[s], W = q.bwords[u], k = __popc(fp.step_mask[s]);
+        for (u32 w0 = warp_from(t, first_warp) * 32u; w0 < W; w0 += t.nwarps() * 32u) {
+            const u32 i = w0 + lane_id();
+            u32 x = 0;
+            if (i < W) {
+                x = q.bm[u][i];
+                for (u32 a = marks; a < marks + k; ++a) {
+                    x &= q.acc[a * q.acc_words + i];
+                    q.acc[a * q.acc_words + i] = 0;
+                }
+                q.bm[u][i] = x;
+            }
+            append_word(g, q, u, i, x);
+        }
+        marks += k;
+        first_warp += (W + 31u) / 32u;
+    }
+    TSYNC_B(t);
+    return true;
+}
+
 // matching/FilterVertices.cpp:841-912 (generateCandidates): candidates of u
 // are the data vertices of u's label, with enough degree and NLF, adjacent to
 // a live candidate of every pivot. The accumulator bitmaps (acc, tmp) are
@@ -628,41 +678,6 @@ __device__ bool step_generate(Team& t, const DevGraph& g, QState& q, u32 u, u32 
     const QDesc* d = q.desc;
     const u32 lu = d->label[u];
     const u32 W = q.bwords[u];
-    if (q.nlf_all) {
-        // Large team: u's NLF set is in bm[u] (stage 1). Two pivots are marked
-        // at a time, and the list keeps the order in which warps append to it
-        // until the filter's end sorts it (no step before depends on it): two
-        // barriers per two pivots, where a pivot took one or two and the ordered
-        // compaction two more (a step with one pivot 18-20 -> 14 us, with two
-        // 26-30 -> 16-18 us).
-        for (u32 pm = pivots; pm;) {
-            const u32 p = (u32)__ffs(pm) - 1;
-            pm &= pm - 1;
-            mark_neighbours(t, g, q, p, lu, q.acc);
-            const bool two = pm != 0;
-            if (two) {
-                mark_neighbours(t, g, q, (u32)__ffs(pm) - 1, lu, q.tmp);
-                pm &= pm - 1;
-            }
-            TSYNC_B(t);
-            for (u32 w0 = t.warp() * 32u; w0 < W; w0 += t.nwarps() * 32u) {
-                const u32 i = w0 + lane_id();
-                u32 x = 0;
-                if (i < W) {
-                    x = q.bm[u][i] & q.acc[i];
-                    q.acc[i] = 0;
-                    if (two) {
-                        x &= q.tmp[i];
-                        q.tmp[i] = 0;
-                    }
-                    q.bm[u][i] = x;
-                }
-                if (!pm) append_word(g, q, u, i, x);
-            }
-            TSYNC_B(t);
-        }
-        return true;
-    }
     bool first = true;
     u32 pm = pivots;
     while (pm) {
@@ -724,13 +739,14 @@ __device__ bool step_generate(Team& t, const DevGraph& g, QState& q, u32 u, u32 
 // whose dead entries have their bit clear), which every later filter step
 // reads through the bitmap, and the filter's last step compacts each pruned
 // vertex once.
+// With `more` the next step belongs to the same group and needs no barrier before it.
 template <class Team>
-__device__ bool step_prune(Team& t, const DevGraph& g, QState& q, u32 u, u32 pivots) {
+__device__ bool step_prune(Team& t, const DevGraph& g, QState& q, u32 u, u32 pivots, u32 first_warp, bool more) {
     const QDesc* d = q.desc;
     const u32 lane = lane_id(), grp = lane >> 3, lg = lane & 7u;
     const u32 base_u = bucket_base(g, d->label[u]);
     const u32 N = q.cnt[u];
-    for (u32 i0 = t.warp() * 4u; i0 < N; i0 += t.nwarps() * 4u) {
+    for (u32 i0 = warp_from(t, first_warp) * 4u; i0 < N; i0 += t.nwarps() * 4u) {
         u32 i = i0 + grp;
         u32 v = i < N ? q.list[u][i] : 0;
         const bool live = i < N && test_bit(q.bm[u], v - base_u);  // the list may hold dead entries
@@ -767,7 +783,7 @@ __device__ bool step_prune(Team& t, const DevGraph& g, QState& q, u32 u, u32 piv
             atomicAnd(q.bm[u] + (pos >> 5), ~(1u << (pos & 31u)));
         }
     }
-    TSYNC_B(t);
+    if (!more) TSYNC_B(t);
     return true;
 }
 
@@ -1466,10 +1482,7 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
         // hands over zero item counts, so the NLF stage depends on nothing here
         // and needs no barrier before it (4-8 us of a preparation).
         if (cfl)
-            for (u32 i = t.rank(); i < q.acc_words; i += t.size()) {
-                q.acc[i] = 0;
-                q.tmp[i] = 0;
-            }
+            for (u32 i = t.rank(); i < q.naccs * q.acc_words; i += t.size()) q.acc[i] = 0;
         if (d->order == PSM_ORDER_CFL)
             for (u32 i = t.rank(); i < PSM_PLAN_WORDS; i += t.size()) q.est_out[i] = 0;
         if (t.rank() == 0) {
@@ -1559,11 +1572,15 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
         j -= 1;
         if (d->filter == PSM_FILTER_GQL) {
             if (j < 2 * n) {  // refine (round j / n) of u = j % n
+                // a vertex reads its neighbours' sets and writes its own: runs of
+                // vertices without an edge between them need no barrier inside
                 const u32 u = j % n;
                 if (!q.empty) {
                     const u32 base = bucket_base(g, d->label[u]);
                     const u32 N = q.cnt[u];
-                    for (u32 i = t.warp(); i < N; i += t.nwarps()) {
+                    u32 at = 0;
+                    while (at < 3u && (d->refine_join >> (j - at) & 1ull)) ++at;
+                    for (u32 i = warp_from(t, at * (t.nwarps() / 4u)); i < N; i += t.nwarps()) {
                         u32 v = q.list[u][i];
                         u32 pos = v - base;
                         if (!test_bit(q.bm[u], pos)) continue;
@@ -1571,6 +1588,7 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
                             atomicAnd(q.bm[u] + (pos >> 5), ~(1u << (pos & 31u)));
                     }
                 }
+                if (j + 1 < 2 * n && (d->refine_join >> (j + 1) & 1ull)) return true;
                 TSYNC_B(t);
                 return true;
             }
@@ -1598,9 +1616,17 @@ __device__ bool run_step(Team& t, const DevGraph& g, QState& q, DevArena* arena,
             return true;
         }
         j -= 1;
-        if (j < fp.nsteps)
-            return fp.step_kind[j] == STEP_GEN ? step_generate(t, g, q, fp.step_u[j], fp.step_mask[j])
-                                               : step_prune(t, g, q, fp.step_u[j], fp.step_mask[j]);
+        if (j < fp.nsteps) {
+            const u32 u = fp.step_u[j], mask = fp.step_mask[j], group = fp.step_group[j];
+            if (fp.step_kind[j] == STEP_PRUNE) {
+                u32 at = 0;  // place in its group: a quarter of the warps further on each
+                while (at < 3u && fp.step_group[j - at] == 0) ++at;
+                const bool more = j + 1 < fp.nsteps && fp.step_group[j + 1] == 0;
+                return step_prune(t, g, q, u, mask, at * (t.nwarps() / 4u), more);
+            }
+            if (!q.nlf_all) return step_generate(t, g, q, u, mask);
+            return group == 0 || generate_group(t, g, q, fp, j, group);
+        }
         j -= fp.nsteps;
     }
     // tail: empty check, tables, order, enumeration plan
@@ -1744,6 +1770,7 @@ __device__ void prepare_query_hybrid(GridTeam& gt, const DevGraph& g, QState& q,
         if (!run_step(gt, g, q, arena, k)) return;
         if (gt.rank() == 0) trace_step(q, k);
         ++k;
+        if (!gt.sync()) return;  // a group's inner steps end without a barrier
     }
 }
 

@@ -19,6 +19,7 @@
 #define PSM_MAXQ 32          // query vertices handled by the kernels
 #define PSM_MAXNLF 1024      // sum over query vertices of distinct neighbour labels
 #define PSM_MAXSTEPS 96      // CFL filter steps per plan (<= 3 per query vertex)
+#define PSM_ACCS 8           // mark bitmaps of the whole-grid team (other teams: 2)
 #define PSM_MAXOPT 3         // start-vertex options kept by the CFL rank heap
 #define PSM_MAXDIR 992       // directed query edges (32 * 31)
 #define PSM_PLAN_WORDS 4096  // CFL order plan blob capacity (u32 words)
@@ -56,6 +57,10 @@ struct FilterPlan {
     u32 step_u[PSM_MAXSTEPS];
     u32 step_kind[PSM_MAXSTEPS];
     u32 step_mask[PSM_MAXSTEPS];  // pivot query vertices as a bitmask
+    // Steps of the group that begins here (0: inside one). A group's steps are
+    // of one kind and none reads what another writes, so they can share their
+    // barriers; a generating group has at most PSM_ACCS pivots in all.
+    u32 step_group[PSM_MAXSTEPS];
 };
 
 // Query descriptor, built on the host, read by the kernels.
@@ -67,6 +72,9 @@ struct QDesc {
     u32 label[PSM_MAXQ];
     u32 deg[PSM_MAXQ];
     u32 adj[PSM_MAXQ];          // neighbour bitmask
+    // GQL refinement: bit s when step s (vertex s mod n, two rounds) is
+    // independent of the steps since the last clear bit
+    u64 refine_join;
     // NLF items: 0..n-1 are the query vertices; n..n+nvirt-1 are the
     // relabelled unit-query vertices whose candidate counts pick the CFL order
     // start vertex (only counted).
@@ -118,9 +126,10 @@ struct QState {
     u32 cnt[PSM_MAXQ];      // candidate counts
     u32 item_cnt[PSM_MAXQ + PSM_MAXOPT];
     u32 nlf_all;            // CFL: stage 1 left every vertex's NLF set in bm (large teams)
-    u32* acc;               // CFL accumulator bitmap (max bwords)
-    u32* tmp;               // CFL per-pivot bitmap
-    u32 acc_words;          // words of acc / tmp
+    u32* acc;               // CFL mark bitmaps: naccs of acc_words words (max bwords)
+    u32* tmp;               // the second of them
+    u32 acc_words;
+    u32 naccs;
     // tables: row counts / offsets for all directed edges, concatenated
     u32* P;                 // [total_rows + 1] absolute offsets into adj
     u32 P_rows;             // rows that P has room for (from the label frequencies)
