@@ -81,7 +81,8 @@ typedef struct psm_result {
     uint64_t tasks;           /* enumeration tasks run (launch-wide)            */
     uint64_t idle_polls;      /* polls of idle warps waiting for work           */
     uint64_t count_internal;  /* embeddings the enumerator counted (unclamped:
-                                 >= count when the cap stopped the query; the
+                                 >= count when the cap stopped the query, by far
+                                 where counted vertices multiply; the
                                  work and alg_bytes above correspond to it) */
 } psm_result;
 
